@@ -10,6 +10,9 @@ namespace tchem_gb {
 
 constexpr int kMaxMechs = 64;       // mechanisms per time-advance call
 constexpr int kMaxGroupSlots = 8;   // structure-compatible mechanisms sharing one launch
+// Status of a sample that the batched sparse-LU kernel leaves to the general kernel of the same call
+// (never seen by the caller).
+constexpr int kStatusRedo = 64;
 constexpr int kTapeSegment = 32;    // steps between trajectory checkpoints (adjoint)
 
 // Byte offsets of the sections of one warp's shared-memory region (mixed form). Kept in the
@@ -17,7 +20,6 @@ constexpr int kTapeSegment = 32;    // steps between trajectory checkpoints (adj
 struct MixedLayout {
   uint32_t warp_bytes;
   uint32_t x, keff, q, x32, keff32, d32, ustage, lrow, pinv, piv, ybuf, vec, stats, red, item;
-  uint32_t lu;   // [nnz] FP32 factors of the sparse-LU shape (else 0)
   uint32_t src;  // [m] the sample's E3SM source term (E3SM instantiations only; else 0)
   int32_t LDU, LDL;
   int32_t simplified;  // 1: simplified-Newton form; 2: full Newton on the Gauss-Jordan inverse; 0: LU
@@ -61,6 +63,8 @@ struct AdvanceParams {
   const double* keff_in;                        // [B][R]
   const double* src_in;                         // [B][m] (src_stride m) or one zero row (src_stride 0)
   int64_t src_stride;
+  // Not null: only the samples with status kStatusRedo, none of them when the count is 0.
+  const int32_t* redo_count;
 };
 
 }  // namespace tchem_gb

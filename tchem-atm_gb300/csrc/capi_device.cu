@@ -14,6 +14,7 @@
 #include "capi_internal.hpp"
 #include "kernels.hpp"
 #include "kernels_mixed.hpp"
+#include "lane_tables.hpp"
 #include "mech_host.hpp"
 
 namespace tchem_gb {
@@ -35,7 +36,16 @@ DeviceTables* tables_for(const tchem_gb_mech* mech, int dev) {
   std::lock_guard<std::mutex> lk(m->mu);
   if (!m->host_tables) m->host_tables.reset(new HostTables(build_host_tables(m->km)));
   if (static_cast<int>(m->device_tables.size()) <= dev) m->device_tables.resize(dev + 1, nullptr);
-  if (!m->device_tables[dev]) m->device_tables[dev] = upload_tables(*m->host_tables, dev);
+  if (!m->device_tables[dev]) {
+    DeviceTables* t = upload_tables(*m->host_tables, dev);
+    try {
+      t->lanes = upload_lane_tables(*m->host_tables, dev, device_info(dev).max_smem_optin);
+    } catch (...) {
+      destroy_device_tables(t);
+      throw;
+    }
+    m->device_tables[dev] = t;
+  }
   return m->device_tables[dev];
 }
 
@@ -153,6 +163,11 @@ struct GroupPlan {
   int threads_per_sample = 32;
   bool tc = false;  // the tensor-core form (kernels_tc_advance.cu)
   MixedLayout ml{};
+  // the batched sparse-LU kernel runs first and leaves single samples to the kernel above
+  int lane_shape = -1;  // -1: not used
+  int lane_grid = 0;
+  LaneSmem lane_smem{};
+  LaneDev lane_dev{};
 };
 
 struct Plan {
@@ -162,6 +177,37 @@ struct Plan {
   size_t bytes = 0;
   int m_max = 0;
 };
+
+// The batched sparse-LU kernel's shape for a batch: the fewest samples per CTA (the most slots per
+// sample, the shortest round) that still hold the batch at once, else the most that one CTA per SM holds
+// (samples then follow each other through the lanes). The shape with two CTAs per SM takes longer per
+// round (51 species: 160 k cycles for 32 samples against 103 k for 16) and less per sample, so it pays
+// when its lanes are filled several times over: from twice its room (5,003 samples over 60 s: 556 ms
+// with one CTA per SM, 618 ms with two).
+void plan_lanes(GroupPlan& g, const DeviceTables& dt, const DeviceInfo& info, int nbatch) {
+  if (!dt.lanes) return;
+  const int fp64 = g.form == TCHEM_GB_FORM_PLAIN_FP64 ? 1 : 0;
+  long best = 0;
+  for (int k = kLaneShapeCount - 1; k >= 0; --k) {
+    if (!dt.lanes->valid[fp64][k]) continue;
+    const LaneShape sh = kLaneShapes[k];
+    const long room = static_cast<long>(info.sm_count) * sh.ctas * sh.S;
+    if (room <= best || (sh.ctas > 1 && nbatch < 2 * room && g.lane_shape >= 0)) continue;
+    best = room;
+    g.lane_shape = k;
+    if (room >= nbatch) break;
+  }
+  if (g.lane_shape < 0) return;
+  const LaneShape sh = kLaneShapes[g.lane_shape];
+  const LaneDev& d = dt.lanes->dev[fp64][g.lane_shape];
+  g.lane_dev = d;
+  g.lane_smem = lane_smem(g.dev.L, d.n_entries, d.n_t, d.table_bytes, sh.S, sh.P(), fp64 != 0);
+  lane_place_streams(g.lane_smem, d, lane_room(sh.ctas, info.max_smem_optin));
+  // the limit, not this plan's bytes: another group or thread may launch the same kernel with more
+  cudaFuncSetAttribute(lane_kernel(g.lane_shape, fp64 != 0), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                       info.max_smem_optin);
+  g.lane_grid = std::min(info.sm_count * sh.ctas, (std::max(nbatch, 1) + sh.S - 1) / sh.S);
+}
 
 // Groups structurally identical mechanisms and sizes each group's launch.
 // e3sm: the E3SM time advance (per-sample rate constants and source terms): every rate form of
@@ -234,14 +280,18 @@ Plan make_plan(const tchem_gb_mech* const* mechs, int n_mechs, int nbatch, bool 
       g.gmat_elems_per_warp = tc_advance_matrix_floats();  // floats per CTA
       g.gmat_offset = off;
       off += up256(sizeof(float) * g.gmat_elems_per_warp * static_cast<size_t>(g.grid));
+      if (o.form == TCHEM_GB_FORM_MIXED || o.form == TCHEM_GB_FORM_MIXED_SIMPLIFIED)
+        plan_lanes(g, *dts[g.mechs[0]], info, nbatch);
       continue;
     }
     if (mixed) {
       int tps = o.threads_per_sample;
       if (tps == 0 && o.form >= 0 && o.form < 3) tps = mechs[g.mechs[0]]->tps_pref[o.form];
+      // full Newton, one warp's worth of threads above 32 species: the batched sparse-LU kernel (the
+      // samples it leaves go to the Gauss-Jordan shape)
+      if (o.form == TCHEM_GB_FORM_MIXED && tps == 32 && L.m > 32 && L.m <= 128 && !e3sm) tps = 0;
       MixedConfig mc = mixed_config(L, tps, info.sm_count, info.max_smem_optin, nbatch,
-                                    o.form == TCHEM_GB_FORM_MIXED_SIMPLIFIED, e3sm,
-                                    g.dev.lu_prog ? g.dev.lu.nnz : 0);
+                                    o.form == TCHEM_GB_FORM_MIXED_SIMPLIFIED, e3sm);
       g.kernel = mc.kernel;
       g.warps_per_block = mc.warps_per_block;
       g.grid = mc.grid;
@@ -250,6 +300,7 @@ Plan make_plan(const tchem_gb_mech* const* mechs, int n_mechs, int nbatch, bool 
       g.ml = mc.ml;
       g.matrix_in_smem = true;
       g.lda = L.m;
+      if (o.form == TCHEM_GB_FORM_MIXED && tps == 0) plan_lanes(g, *dts[g.mechs[0]], info, nbatch);
       continue;
     }
     g.lda = L.m | 1;
@@ -276,6 +327,7 @@ Plan make_plan(const tchem_gb_mech* const* mechs, int n_mechs, int nbatch, bool 
       g.gmat_offset = off;
       off += up256(sizeof(double) * g.gmat_elems_per_warp * static_cast<size_t>(g.grid) * W);
     }
+    plan_lanes(g, *dts[g.mechs[0]], info, nbatch);
   }
   plan.bytes = off;
   return plan;
@@ -403,7 +455,7 @@ int time_advance_impl(const tchem_gb_mech* const* mechs, int n_mechs, const int3
   int32_t* error_word = reinterpret_cast<int32_t*>(ws + 64);
   int32_t* counts = reinterpret_cast<int32_t*>(ws + 128);
   cudaError_t e = cudaMemsetAsync(ws, 0, 64, stream);  // queues (the error word persists until read)
-  if (e == cudaSuccess) e = cudaMemsetAsync(ws + 128, 0, 64, stream);
+  if (e == cudaSuccess) e = cudaMemsetAsync(ws + 128, 0, 192, stream);
   if (e != cudaSuccess) return cuda_fail(e, "cudaMemsetAsync(workspace)");
   int32_t* items = plan.need_items ? reinterpret_cast<int32_t*>(ws + plan.items_offset) : nullptr;
   if (plan.need_items) {
@@ -478,6 +530,19 @@ int time_advance_impl(const tchem_gb_mech* const* mechs, int n_mechs, const int3
     P.keff_in = rates.keff;
     P.src_in = rates.src;
     P.src_stride = rates.src_stride;
+    if (gp.lane_shape >= 0) {
+      LaneParams LP{};
+      LP.a = P;
+      LP.p = gp.lane_dev;
+      LP.s = gp.lane_smem;
+      LP.redo_count = counts + 16 + g;
+      e = launch_lanes(LP, gp.lane_shape, gp.form == TCHEM_GB_FORM_PLAIN_FP64, gp.lane_grid, gs);
+      if (e != cudaSuccess) return cuda_fail(e, "time-advance kernel launch");
+      note_launch();
+      // the samples it left, if any: the general kernel, on a queue of its own
+      P.redo_count = LP.redo_count;
+      P.queue = queue + 64 + g;
+    }
     if (gp.tc)
       e = launch_trbdf2_tc(P, gp.grid, gp.smem, gs);
     else if (gp.form == TCHEM_GB_FORM_MIXED || gp.form == TCHEM_GB_FORM_MIXED_SIMPLIFIED)

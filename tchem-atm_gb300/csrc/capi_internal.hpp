@@ -13,8 +13,9 @@
 namespace tchem_gb {
 
 // Workspace header: work-queue heads at byte 0 (16 x int32), the device error word at 64
-// (read and cleared by tchem_gb_device_error), group counts at 128.
-constexpr size_t kHeaderBytes = 256;
+// (read and cleared by tchem_gb_device_error), group counts at 128; of the samples that the batched
+// kernel leaves to the general one, the counts at 192 and the work-queue heads at 256 (16 x int32 each).
+constexpr size_t kHeaderBytes = 512;
 
 struct DeviceInfo {
   int sm_count = 0;

@@ -125,7 +125,7 @@ extern "C" int tchem_gb_time_advance_noalloc(const tchem_gb_mech* const* mechs, 
     return TCHEM_GB_ERR_ARG;
   }
   // queue heads, device error word and group counts start at zero
-  e = cudaMemsetAsync(scratch, 0, 256, static_cast<cudaStream_t>(stream_v));
+  e = cudaMemsetAsync(scratch, 0, tchem_gb::kHeaderBytes, static_cast<cudaStream_t>(stream_v));
   if (e != cudaSuccess) {
     set_last_error(std::string("tchem_gb_time_advance_noalloc: cudaMemsetAsync: ") + cudaGetErrorString(e));
     return TCHEM_GB_ERR_CUDA;

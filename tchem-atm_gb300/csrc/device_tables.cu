@@ -10,6 +10,8 @@
 #include <stdexcept>
 #include <string>
 
+#include "lane_tables.hpp"
+
 namespace tchem_gb {
 
 namespace {
@@ -286,7 +288,6 @@ HostTables build_host_tables(const KineticModel& km) {
   L.off_rf_sp = sec(sizeof(int16_t) * rf_sp.size());
   L.off_pr_r = sec(sizeof(int16_t) * pr_r.size());
   L.off_jc_f = sec(sizeof(int16_t) * jc_f.size());
-  L.off_js_e = -1;
   L.blob_bytes = static_cast<int32_t>(align16(off));
   ht.blob.assign(L.blob_bytes, 0);
   put(ht.blob, L.off_emis, emis);
@@ -312,22 +313,14 @@ HostTables build_host_tables(const KineticModel& km) {
     std::vector<int32_t> wids(m);
     for (int k = 0; k < m; ++k) wids[k] = k;
     const Sliced js = make_slices(jlists, jids, static_cast<int16_t>(L.NF));
-    // sparse-LU entry of every Jacobian slot (padding lanes: 0, never written)
-    std::vector<int16_t> js_e;
     if (m <= kSparseLuMaxSpecies) {
       std::vector<std::pair<int, int>> nz;
       for (const auto& kv : jac) nz.push_back(kv.first);
       try {
         ht.slu = build_sparse_lu(m, nz);
       } catch (const std::exception&) {
-        ht.slu = SparseLuHost{};  // no program: the sparse-LU shapes are not offered
+        ht.slu = SparseLuHost{};  // too many entries for the program encoding
       }
-      if (ht.slu.lay.m == m)
-        for (int32_t rc : js.item) {
-          int e = 0;
-          if (rc >= 0) e = ht.slu.entry[static_cast<size_t>(ht.slu.pos[rc >> 16]) * m + ht.slu.pos[rc & 0xffff]];
-          js_e.push_back(static_cast<int16_t>(e));
-        }
     }
     const Sliced ws = make_slices(per_species, wids, static_cast<int16_t>(R));
     std::vector<float> jse_nu32(js.val.begin(), js.val.end());
@@ -352,7 +345,6 @@ HostTables build_host_tables(const KineticModel& km) {
     X.off_rf_sp = sx(sizeof(int16_t) * rf_sp.size());
     X.off_jse_f = sx(sizeof(int16_t) * js.idx.size());
     X.off_wse_r = sx(sizeof(int16_t) * ws.idx.size());
-    X.off_js_e = js_e.empty() ? -1 : sx(sizeof(int16_t) * js_e.size());
     // CSR sections are not part of the mixed blob
     X.off_pr_ptr = X.off_pr_r = X.off_pr_nu = X.off_jz_rc = X.off_jz_ptr = X.off_jc_f = X.off_jc_nu = X.off_jc_nu32 = -1;
     X.blob_bytes = static_cast<int32_t>(align16(o));
@@ -370,7 +362,6 @@ HostTables build_host_tables(const KineticModel& km) {
     put(ht.blob_x, X.off_ws_off, ws.off);
     put(ht.blob_x, X.off_wse_r, ws.idx);
     put(ht.blob_x, X.off_wse_nu, ws.val);
-    if (!js_e.empty()) put(ht.blob_x, X.off_js_e, js_e);
   }
 
   // Structural signature: everything except the rate parameters.
@@ -405,7 +396,6 @@ DeviceTables* upload_tables(const HostTables& ht, int device) {
   const size_t o_e3a = sec(sizeof(int32_t) * std::max<size_t>(1, ht.e3_adj_sp.size()));
   const size_t o_e3o = sec(sizeof(int32_t) * std::max<size_t>(1, ht.e3_o1d.size()));
   const size_t o_e3op = sec(sizeof(double) * std::max<size_t>(1, ht.e3_o1d_par.size()));
-  const size_t o_lu = sec(sizeof(int32_t) * std::max<size_t>(1, ht.slu.prog.size()));
   std::vector<unsigned char> host(off, 0);
   std::memcpy(host.data() + o_blob, ht.blob.data(), ht.blob.size());
   std::memcpy(host.data() + o_blob_x, ht.blob_x.data(), ht.blob_x.size());
@@ -425,8 +415,6 @@ DeviceTables* upload_tables(const HostTables& ht, int device) {
   if (!ht.e3_o1d.empty()) std::memcpy(host.data() + o_e3o, ht.e3_o1d.data(), sizeof(int32_t) * ht.e3_o1d.size());
   if (!ht.e3_o1d_par.empty())
     std::memcpy(host.data() + o_e3op, ht.e3_o1d_par.data(), sizeof(double) * ht.e3_o1d_par.size());
-  if (!ht.slu.prog.empty())
-    std::memcpy(host.data() + o_lu, ht.slu.prog.data(), sizeof(int32_t) * ht.slu.prog.size());
 
   int prev = 0;
   cudaGetDevice(&prev);
@@ -467,8 +455,6 @@ DeviceTables* upload_tables(const HostTables& ht, int device) {
   t->dev.e3_o1d_par = reinterpret_cast<const double*>(b + o_e3op);
   t->dev.e3_no1d = static_cast<int32_t>(ht.e3_o1d.size() / 7);
   t->dev.M_index = ht.M_index;
-  t->dev.lu_prog = ht.slu.prog.empty() ? nullptr : reinterpret_cast<const int32_t*>(b + o_lu);
-  t->dev.lu = ht.slu.lay;
   t->dev_x = t->dev;
   t->dev_x.L = ht.Lx;
   t->dev_x.blob = b + o_blob_x;
@@ -477,6 +463,7 @@ DeviceTables* upload_tables(const HostTables& ht, int device) {
 
 void destroy_device_tables(DeviceTables* t) {
   if (!t) return;
+  destroy_lane_tables(t->lanes);
   if (t->allocation) {
     int prev = 0;
     cudaGetDevice(&prev);

@@ -49,9 +49,6 @@ struct MechLayout {
   int32_t NJS, NJE, NWS, NWE;
   int32_t off_js_rc, off_js_cnt, off_js_off, off_jse_f, off_jse_nu32;  // Jacobian nonzeros
   int32_t off_ws_sp, off_ws_cnt, off_ws_off, off_wse_r, off_wse_nu;    // net production per species
-  // Sparse-LU shape (m <= kSparseLuMaxSpecies, else -1): per Jacobian slot of the sliced-ELL
-  // program (off_js_rc), the entry of (row, col) in the static-order filled pattern (int16).
-  int32_t off_js_e;
 };
 
 // Device pointers of one mechanism on one device (passed by value to kernels).
@@ -80,9 +77,6 @@ struct MechDev {
   const int32_t* e3_o1d;      // [e3_no1d][7]: reactions 1..3, photolysis reaction, species 1..3
   const double* e3_o1d_par;   // [e3_no1d][6]: A1, C1, A2, C2, A3, C3
   int32_t e3_no1d, M_index;
-  // Static-order sparse LU program (sparse_lu.hpp), or null when the mechanism is too large.
-  const int32_t* lu_prog;
-  SparseLuLayout lu;
 };
 
 // Host-side packed tables, built from a parsed kinetic model.
@@ -91,7 +85,7 @@ struct HostTables {
   std::vector<unsigned char> blob;
   MechLayout Lx{};                 // mixed form (sliced-ELL programs)
   std::vector<unsigned char> blob_x;
-  SparseLuHost slu;                // sparse-LU program (slu.lay.m == 0: none)
+  SparseLuHost slu;                // static-order sparse LU of tchem_gb_mech_sparse_lu (slu.lay.m == 0: none)
   std::vector<int32_t> rate_type, conv_exp, cf_ptr, cf_idx;
   std::vector<double> rate_param;
   std::vector<int32_t> rx_sidx, rx_n;  // stoichiometry by reaction (MechDev::rx_*)
@@ -114,11 +108,14 @@ struct HostTables {
 
 HostTables build_host_tables(const KineticModel& km);
 
+struct LaneTables;  // instruction streams of the batched sparse-LU kernel (lane_tables.cu)
+
 struct DeviceTables {
   int device = -1;
   MechDev dev{};    // plain-form tables
   MechDev dev_x{};  // mixed-form tables (same rate parameters, sliced-ELL blob)
   void* allocation = nullptr;
+  LaneTables* lanes = nullptr;  // null: the mechanism does not fit the encoding
 };
 
 DeviceTables* upload_tables(const HostTables& ht, int device);

@@ -32,6 +32,7 @@ size_t fp64_warp_smem_bytes(const MechLayout& L, int lda, bool matrix_in_smem, b
 
 template <int NPL>
 __global__ void __launch_bounds__(256, 1) trbdf2_fp64_kernel(const __grid_constant__ AdvanceParams P) {
+  if (P.redo_count && *P.redo_count == 0) return;
   extern __shared__ __align__(128) unsigned char smem[];
   uint64_t* mbar = reinterpret_cast<uint64_t*>(smem);
   unsigned char* tables = smem + 16;
@@ -79,6 +80,7 @@ __global__ void __launch_bounds__(256, 1) trbdf2_fp64_kernel(const __grid_consta
     item = __shfl_sync(kFullMask, item, 0);
     if (item >= n_items) break;
     const int s = P.items ? P.items[item] : item;
+    if (P.redo_count && P.status[s] != kStatusRedo) continue;  // advanced by the batched kernel
     const tchem_gb_tadv ta = P.tadv[s];
     if (P.t_out[s] >= ta.tend) {
       if (lane == 0) {

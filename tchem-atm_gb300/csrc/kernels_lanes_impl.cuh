@@ -1,0 +1,1203 @@
+// Batched TR-BDF2 kernel over a static-order sparse LU.
+//
+// A CTA advances S samples in step, one Newton iteration of each per round; every shared-memory
+// array has the sample as its fastest index. A warp's 32 lanes are S samples x 32 / S slots, and the
+// slots share the work of a round by the mechanism's instruction streams (lane_program.hpp): rates
+// and species are dealt to the slots and live in registers, the matrix, the factorization and the
+// triangular solves are streams of 16-byte packets read ahead from global memory (L1 / L2), the same
+// for every sample, with a CTA barrier at the end of each level of the elimination schedule; the
+// nearly dense trailing block is inverted in registers, a 2-D grid of slots each holding a tile.
+//
+// Each sample is at its own step, stage and iteration; what differs is decided once per round by one
+// warp from the reduced norms and handed to the slots as a code per sample. A sample that ends
+// hands its lane to the next one of the work queue. The right-hand side at a converged stage is the
+// one the next round evaluates anyway (the next stage or step starts there), so a Newton iteration
+// costs one right-hand side: f(y_n), f(y_gamma) and f(y_{n+1}) need no evaluations of their own.
+//
+// Why: the dense kernels spend 44 k (LU) to 140 k (Gauss-Jordan) products on a 51-species matrix whose
+// sparse factors need 7.8 k, and every index of a sparse factorization costs as much as its product when
+// one warp works on one sample. What bounds this one: chains of dependent shared-memory loads and FP64
+// instructions (2 per cycle and SM) between barriers, 34 k cycles per round with one sample on the SM,
+// 103 k with 16. Measured against the dense kernels (one GB300): 51 species, one sample over 60 s 92 to
+// 56 ms, 4,096 samples over 3,600 s 1.20 to 1.04 s (FP32), 300 samples over 0.1 s 1.01 to 0.20 s (FP64);
+// 120 species, 257 samples over 1 s 440 to 238 ms; 300 species, 24 samples over 1e-4 s 442 to 65 ms (the
+// blocked LU on tensor cores with the matrix in L2); E3SM, 2,000 columns over 1,800 s 117 to 8.6 ms (FP64).
+//
+// T = float: the full-Newton FP32 form (FP32 matrix, factors and solves, FP64 residual, one
+// refinement sweep with an FP64 Jacobian-vector product per solve). T = double: the plain form.
+// A sample whose factorization meets a zero, non-finite or small pivot (a multiplier above
+// kLaneMaxGrowth), or that asks for something outside this kernel, is left untouched with status
+// kStatusRedo and advanced by the general kernel, which pivots.
+#pragma once
+
+#include <cuda_runtime.h>
+
+#include <cstdint>
+
+#include "engine.cuh"
+#include "kernels_lanes.hpp"
+#include "lane_program.hpp"
+
+namespace tchem_gb {
+namespace lanes {
+
+// Largest multiplier |l_ik| accepted without pivoting. The diagonal of I - c J is 1 + c x (loss
+// rate), and a column's off-diagonal entries are c x (loss rate) x yield, so multipliers stay near
+// the yields (about 1); partial pivoting would bound them by 1.
+constexpr float kLaneMaxGrowth = 64.f;
+constexpr int kLaneMaxGrowthHi = 0x40500000;  // the high word of 64.0
+
+// Control block: doubles then ints, each [S].
+enum CtlD { D_T, D_DT, D_TEND, D_DTMIN, D_DTMAX, D_COEF, D_COUNT };
+enum CtlI { I_SMP, I_CODE, I_LAST, I_ITER, I_MAXITER, I_NEWT, I_MAXNEWT, I_TRY, I_STAGE, I_BAD, I_STEPS, I_REJ, I_NFAIL,
+            I_NITS, I_NOK0, I_NATT, I_STATUS, I_ACC, I_COUNT,
+            I_SLOT = I_LAST };  // the mechanism slot is needed only until the first step begins
+enum Code {
+  C_ITER = 0,     // next Newton iteration of the same stage
+  C_STAGE = 1,    // stage 1 converged: stage 2 starts at y_gamma
+  C_STEP = 2,     // stage 2 converged: error test
+  C_RETRY = 3,    // Newton failed: the step starts again with half the step size
+  C_IDLE = 4,     // no sample
+  C_FRESH = 5,    // new sample
+  C_ACCEPT = 6,   // step accepted, the next one starts
+  C_REJECT = 7,   // step rejected
+  C_DONE = 8      // finished: write the outputs
+};
+
+static_assert(D_COUNT == kLaneControlDoubles && I_COUNT == kLaneControlInts, "control block size");
+
+template <typename T>
+struct Num;
+template <>
+struct Num<float> {
+  // hardware reciprocal (1 ulp): the factors are refined against an FP64 residual
+  static __device__ __forceinline__ float recip(float v) {
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(v));
+    return r;
+  }
+  static __device__ __forceinline__ float mul_sub(float a, float b, float c) { return fmaf(-a, b, c); }
+};
+template <>
+struct Num<double> {
+  // Newton-Raphson on the hardware's approximate reciprocal: each pass squares its relative error
+  // (2^-20 at worst), the last one in residual form. A short dependent chain; zero, infinite and NaN
+  // pivots give NaN or 0, which the caller rejects.
+  static __device__ __forceinline__ double recip(double v) {
+    double r;
+    asm volatile("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(v));
+    r = fma(fma(-v, r, 1.0), r, r);
+    r = fma(fma(-v, r, 1.0), r, r);
+    return r;
+  }
+  static __device__ __forceinline__ double mul_sub(double a, double b, double c) { return fma(-a, b, c); }
+};
+
+// Shared memory by 32-bit address: the sections' places are run-time values, and an address in the
+// generic window would cost 64-bit arithmetic for each of a packet's eight operands.
+template <typename T>
+struct Shared {
+  uint32_t at;
+  __device__ __forceinline__ T load(uint32_t index) const;
+  __device__ __forceinline__ void store(uint32_t index, T v) const;
+};
+template <>
+__device__ __forceinline__ float Shared<float>::load(uint32_t index) const {
+  float v;
+  asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(at + 4u * index));
+  return v;
+}
+template <>
+__device__ __forceinline__ void Shared<float>::store(uint32_t index, float v) const {
+  asm volatile("st.shared.f32 [%0], %1;" ::"r"(at + 4u * index), "f"(v) : "memory");
+}
+template <>
+__device__ __forceinline__ double Shared<double>::load(uint32_t index) const {
+  double v;
+  asm volatile("ld.shared.f64 %0, [%1];" : "=d"(v) : "r"(at + 8u * index));
+  return v;
+}
+template <>
+__device__ __forceinline__ void Shared<double>::store(uint32_t index, double v) const {
+  asm volatile("st.shared.f64 [%0], %1;" ::"r"(at + 8u * index), "d"(v) : "memory");
+}
+__device__ __forceinline__ uint4 load_packet(uint32_t at) {
+  uint4 v;
+  asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(at));
+  return v;
+}
+__device__ __forceinline__ uint32_t load_byte(uint32_t at) {
+  uint32_t v;
+  asm volatile("ld.shared.u8 %0, [%1];" : "=r"(v) : "r"(at));
+  return v;
+}
+
+template <typename T, int S, int W>
+struct Kernel {
+  static constexpr int NT = 32 * W;
+  static constexpr int SPW = 32 / S;  // slots per warp
+  static constexpr int P = NT / S;    // slots
+  static constexpr bool kRefine = sizeof(T) == 4;
+  static constexpr int kPair = sizeof(T) == 4 ? 2 : 1;  // rounds of the factor stream worked on at a time
+  static constexpr int NPS = lane_species(P), NRS = lane_reactions(P);
+
+  const LaneParams& K;
+  unsigned char* sm;
+  int s, sl, slot, warp;  // sample, slot in the warp, slot, warp
+  int bad;
+
+  __device__ __forceinline__ uint32_t base() const { return static_cast<uint32_t>(__cvta_generic_to_shared(sm)); }
+  __device__ __forceinline__ Shared<T> lus() const { return Shared<T>{base() + K.s.lu + s * static_cast<uint32_t>(sizeof(T))}; }
+  __device__ __forceinline__ T* lu() const { return reinterpret_cast<T*>(sm + K.s.lu) + s; }
+  __device__ __forceinline__ double* xs() const { return reinterpret_cast<double*>(sm + K.s.x) + s; }
+  __device__ __forceinline__ double* vs() const { return reinterpret_cast<double*>(sm + K.s.v) + s; }
+  // the iterate in T precision: in v's place until v is written (T = double: x itself)
+  __device__ __forceinline__ T* xt() const { return reinterpret_cast<T*>(sm + (kRefine ? K.s.v : K.s.x)) + s; }
+  __device__ __forceinline__ double* qs() const { return reinterpret_cast<double*>(sm + K.s.q) + s; }
+  __device__ __forceinline__ T* ds() const { return reinterpret_cast<T*>(sm + K.s.q) + s; }  // while q is not needed
+  __device__ __forceinline__ Shared<double> xsh() const { return Shared<double>{base() + K.s.x + s * 8u}; }
+  __device__ __forceinline__ Shared<double> qsh() const { return Shared<double>{base() + K.s.q + s * 8u}; }
+  __device__ __forceinline__ double& cd(int k, int smp) const {
+    return reinterpret_cast<double*>(sm + K.s.ctl)[k * S + smp];
+  }
+  __device__ __forceinline__ int& ci(int k, int smp) const {
+    return reinterpret_cast<int*>(sm + K.s.ctl + D_COUNT * S * sizeof(double))[k * S + smp];
+  }
+  __device__ __forceinline__ int& flag(int k) const {
+    return reinterpret_cast<int*>(sm + K.s.ctl + S * (D_COUNT * sizeof(double) + I_COUNT * sizeof(int)))[k];
+  }
+  __device__ __forceinline__ int m() const { return K.a.mech.L.m; }
+
+  // This slot's packets of a stream, a warp's rounds SPW apart: in shared memory where it is resident.
+  __device__ __forceinline__ const uint4* packets(int id, int& rounds) const {
+    const int2 w = reinterpret_cast<const int2*>(sm + K.s.prog)[id * W + warp];
+    rounds = w.y;
+    return (K.s.stream[id] ? reinterpret_cast<const uint4*>(sm + K.s.stream[id]) : K.p.packets[id]) + w.x + sl;
+  }
+
+  // The rounds of one stream in order, two at a time, each pair read while the one before it is
+  // worked on. A stream that is not resident goes through shared memory in chunks: every warp copies
+  // its own packets (cp.async) into its part of [buf, buf + bytes), one half while it reads the other,
+  // so that the warp waits once per chunk for L2 and not once per pair.
+  struct Reader {
+    const uint4* src;       // staged: the next packets to copy; read from global memory: the next packet
+    uint32_t p, buf;        // shared addresses: the next packet, the warp's chunks
+    int cap, left, in_chunk, half;
+    bool global;
+    uint4 a, b;
+  };
+  __device__ __forceinline__ void fetch(Reader& r) const {
+    const int n = min(r.cap, r.left) * SPW, lane = threadIdx.x & 31;
+    const uint32_t dst = r.buf + r.half * r.cap * SPW * 16;
+    for (int i = lane; i < n; i += 32)
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + 16 * i), "l"(r.src + i) : "memory");
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    r.src += r.cap * SPW;
+    r.left -= r.cap;
+    r.half ^= 1;
+  }
+  __device__ __forceinline__ void next_chunk(Reader& r) const {
+    __syncwarp();  // every lane has read the half that is filled now
+    if (r.left > 0) {
+      fetch(r);
+      asm volatile("cp.async.wait_group 1;" ::: "memory");
+    } else {
+      r.half ^= 1;
+      asm volatile("cp.async.wait_group 0;" ::: "memory");
+    }
+    __syncwarp();
+    r.p = r.buf + (r.half * r.cap * SPW + sl) * 16;
+    r.in_chunk = r.cap;
+  }
+  template <int N>
+  __device__ __forceinline__ void read(Reader& r) const {
+    if (r.global) {
+      r.a = __ldg(r.src);
+      if (N == 2) r.b = __ldg(r.src + SPW);
+    } else {
+      r.a = load_packet(r.p);
+      if (N == 2) r.b = load_packet(r.p + SPW * 16);
+    }
+  }
+  template <int N>
+  __device__ __forceinline__ Reader open(int id, uint2 chunk, int& rounds) const {
+    Reader r;
+    const int2 w = reinterpret_cast<const int2*>(sm + K.s.prog)[id * W + warp];
+    rounds = w.y;
+    r.cap = static_cast<int>(chunk.y / (2 * W * SPW * 16)) & ~1;
+    r.in_chunk = 1 << 30;
+    r.global = false;
+    r.src = K.p.packets[id] + w.x;
+    if (K.s.stream[id]) {
+      r.p = base() + K.s.stream[id] + (w.x + sl) * 16;
+    } else if (r.cap >= 2) {
+      r.buf = base() + chunk.x + warp * 2 * r.cap * SPW * 16;
+      r.left = rounds;
+      r.half = 0;
+      fetch(r);
+      next_chunk(r);
+    } else {
+      r.global = true;
+      r.src += sl;
+    }
+    read<N>(r);
+    return r;
+  }
+  // The next N rounds (beyond the last, what is read is not used; the streams end with a spare pair).
+  template <int N>
+  __device__ __forceinline__ void advance(Reader& r) const {
+    r.p += N * SPW * 16;
+    if (r.global) r.src += N * SPW;
+    r.in_chunk -= N;
+    if (r.in_chunk <= 0) next_chunk(r);
+    read<N>(r);
+  }
+  // Shared memory that a stream's chunks may use: what the streams' placement left, or sections whose
+  // contents are not needed at that time.
+  __device__ __forceinline__ uint2 chunk_space(uint32_t off, uint32_t end) const {
+    return K.s.stage_bytes >= end - off ? make_uint2(K.s.stage, K.s.stage_bytes) : make_uint2(off, end - off);
+  }
+
+  // Factor and substitution packets: the entry minus three products, times a pivot's reciprocal (the one
+  // entry where nothing scales it), or the reciprocal of a pivot.
+  template <int PAIR>
+  __device__ __forceinline__ void run_lu(int id, uint2 chunk) {
+    const Shared<T> A = lus();
+    uint32_t rounds = base() + K.s.prog + K.p.level_at[id] + warp;
+    const int levels = K.p.levels[id];
+    if (levels == 0) return;
+    int total, n = static_cast<int>(load_byte(rounds));
+    Reader r = open<PAIR>(id, chunk, total);
+#pragma unroll 1
+    for (int lv = 0; lv < levels; ++lv) {
+      rounds += lv + 1 < levels ? W : 0;
+      const int next = static_cast<int>(load_byte(rounds));
+#pragma unroll 1
+      for (; n > 0; n -= PAIR) {
+        if constexpr (PAIR == 2)
+          packet_pair(A, r);
+        else
+          packet(A, r);
+      }
+      n = next;
+      __syncthreads();
+    }
+  }
+  // FP32 factor: two packets with all their operands read first, so that a level costs one chain of
+  // dependent loads; no branches, unused places multiply zeros.
+  __device__ __forceinline__ void packet_pair(Shared<T> A, Reader& r) {
+    const uint4 w0 = r.a, w1 = r.b;
+    const uint32_t d0 = (w0.x & 0x7fffu) * S, d1 = (w1.x & 0x7fffu) * S;
+    const T e0 = A.load(d0), e1 = A.load(d1);
+    const T a0 = A.load((w0.y & 0xffffu) * S), b0 = A.load((w0.y >> 16) * S);
+    const T a1 = A.load((w0.z & 0xffffu) * S), b1 = A.load((w0.z >> 16) * S);
+    const T a2 = A.load((w0.w & 0xffffu) * S), b2 = A.load((w0.w >> 16) * S);
+    const T s0 = A.load(((w0.x >> LP_SCALE_SHIFT) & 511u) * S);
+    const T f0 = A.load((w1.y & 0xffffu) * S), g0 = A.load((w1.y >> 16) * S);
+    const T f1 = A.load((w1.z & 0xffffu) * S), g1 = A.load((w1.z >> 16) * S);
+    const T f2 = A.load((w1.w & 0xffffu) * S), g2 = A.load((w1.w >> 16) * S);
+    const T s1 = A.load(((w1.x >> LP_SCALE_SHIFT) & 511u) * S);
+    advance<2>(r);
+    T u = Num<T>::mul_sub(a2, b2, Num<T>::mul_sub(a1, b1, Num<T>::mul_sub(a0, b0, e0)));
+    T v = Num<T>::mul_sub(f0, g0, (w1.x & LP_CONT) ? u : e1);
+    v = Num<T>::mul_sub(f2, g2, Num<T>::mul_sub(f1, g1, v));
+    A.store(d0, finish(w0.x, u * s0, u, Num<T>::recip(u)));
+    A.store(d1, finish(w1.x, v * s1, v, Num<T>::recip(v)));
+  }
+  __device__ __forceinline__ T finish(uint32_t h, T scaled, T acc, T inverse) {
+    const T v = (h & LP_PIVOT) ? inverse : scaled;
+    if ((h & LP_PIVOT) && (!(fabs(acc) > T(0)) || !(fabs(v) > T(0)))) bad = 1;  // zero, infinite or NaN
+    if ((h & LP_LCOL) && !(fabs(v) <= T(kLaneMaxGrowth))) bad = 1;
+    return v;
+  }
+  // One packet. FP64: an instruction takes 16 cycles of the SM's pipe whatever its lanes do with it, so
+  // a warp leaves out what none of its slots needs (volatile: the compiler must not compute both sides
+  // and select). FP32 (substitutions): no branches; unused places multiply zeros.
+  __device__ __forceinline__ void packet(Shared<T> A, Reader& r) {
+    const uint4 w = r.a;
+    const uint32_t dst = (w.x & 0x7fffu) * S;
+    T acc = A.load(dst);
+    const T a0 = A.load((w.y & 0xffffu) * S), b0 = A.load((w.y >> 16) * S);
+    const T a1 = A.load((w.z & 0xffffu) * S), b1 = A.load((w.z >> 16) * S);
+    const T a2 = A.load((w.w & 0xffffu) * S), b2 = A.load((w.w >> 16) * S);
+    const T scale = A.load(((w.x >> LP_SCALE_SHIFT) & 511u) * S);
+    advance<1>(r);
+    if constexpr (sizeof(T) == 4) {
+      A.store(dst, scale * Num<T>::mul_sub(a2, b2, Num<T>::mul_sub(a1, b1, Num<T>::mul_sub(a0, b0, acc))));
+    } else {
+      const uint32_t any = __shfl_sync(kFullMask, w.x, 0);  // the warp's flags, as a uniform value
+      if (any & LP_ONE) acc_product(acc, a0, b0);
+      if (any & LP_TWO) acc_product(acc, a1, b1);
+      if (any & LP_THREE) acc_product(acc, a2, b2);
+      T v = acc;
+      if (any & LP_SCALED) asm volatile("mul.rn.f64 %0, %0, %1;" : "+d"(v) : "d"(scale));
+      if (any & LP_PIVOTS) {
+        const T p = Num<T>::recip(acc);
+        if (w.x & LP_PIVOT) {
+          v = p;
+          if (!(fabs(acc) > T(0)) || !(fabs(v) > T(0))) bad = 1;
+        }
+      }
+      // the size as the high word of |v| (monotonic): below 64, and neither infinite nor NaN
+      if ((w.x & LP_LCOL) && (__double2hiint(static_cast<double>(v)) & 0x7fffffff) > kLaneMaxGrowthHi) bad = 1;
+      A.store(dst, v);
+    }
+  }
+  static __device__ __forceinline__ void acc_product(double& acc, double a, double b) {
+    asm volatile("{\n .reg .f64 t;\n neg.f64 t, %1;\n fma.rn.f64 %0, t, %2, %0;\n}" : "+d"(acc) : "d"(a), "d"(b));
+  }
+
+  // In-place Gauss-Jordan inverse of the tail block, no pivot search, two pivots per step: slot (pr, pc) of
+  // the grid holds rows pr + GR a and columns pc + GC c in registers. Per step the owners of the two
+  // pivot rows and columns publish them (double-buffered, one barrier); every slot solves the 2 x 2
+  // pivot block for its columns and updates its tile with both rows. A step is bound by its chain of
+  // barrier, loads and reciprocals and by the instructions around the products: two pivots share them.
+  template <int TR>
+  __device__ __forceinline__ void invert_tail() {
+    constexpr int GR = lane_grid_rows(P), GC = lane_grid_cols(P), F = GR / GC, N = TR * GR, TC = N / GC;
+    constexpr int ST = lane_tail_stride(P, N);
+    const Shared<T> A{lus().at + K.p.tail * S * static_cast<uint32_t>(sizeof(T))};
+    // [2]: two rows, two columns, each [N][S]
+    const Shared<T> pub{base() + K.s.q + s * static_cast<uint32_t>(sizeof(T))};
+    const int pr = slot / GC, pc = slot % GC;
+    T t[TR][TC];
+#pragma unroll
+    for (int a = 0; a < TR; ++a)
+#pragma unroll
+      for (int c = 0; c < TC; ++c) t[a][c] = A.load(((pr + GR * a) * ST + pc + GC * c) * S);
+    if (pr < 2)
+#pragma unroll
+      for (int c = 0; c < TC; ++c) pub.store((pr * N + pc + GC * c) * S, t[0][c]);
+    if (pc < 2)
+#pragma unroll
+      for (int a = 0; a < TR; ++a) pub.store(((2 + pc) * N + pr + GR * a) * S, t[a][0]);
+    __syncthreads();
+#pragma unroll
+    for (int blk = 0; blk < TR * F; ++blk) {
+      const int ta = blk / F, tc = blk, r0 = GC * (blk % F);  // the pivots' tile row and column, first grid row
+#pragma unroll 1
+      for (int b = 0; b < GC; b += 2) {
+        const int k = GC * blk + b;
+        constexpr uint32_t kStep = N * S * static_cast<uint32_t>(sizeof(T));
+        const Shared<T> x0{pub.at + ((k >> 1) & 1) * 4 * kStep}, x1{x0.at + kStep}, y0{x1.at + kStep}, y1{y0.at + kStep};
+        // [a b; c d] = [1 0; l 1] [a b; 0 e]
+        const T pa = x0.load(k * S), pb = x0.load((k + 1) * S), pcc = x1.load(k * S), pd = x1.load((k + 1) * S);
+        const T p0 = Num<T>::recip(pa), l = pcc * p0, w = pb * p0, e = Num<T>::mul_sub(l, pb, pd), p1 = Num<T>::recip(e);
+        T q0[TC], q1[TC], l0[TR], l1[TR], big0 = T(0), big1 = T(0);
+#pragma unroll
+        for (int c = 0; c < TC; ++c) {
+          const T u = x0.load((pc + GC * c) * S), v = x1.load((pc + GC * c) * S);
+          q1[c] = p1 * Num<T>::mul_sub(l, u, v);
+          q0[c] = Num<T>::mul_sub(w, q1[c], p0 * u);
+        }
+#pragma unroll
+        for (int a = 0; a < TR; ++a) {
+          l0[a] = y0.load((pr + GR * a) * S);
+          l1[a] = y1.load((pr + GR * a) * S);
+          big0 = fmax(big0, fabs(l0[a]));
+          big1 = fmax(big1, fabs(Num<T>::mul_sub(l0[a], w, l1[a])));  // after the first elimination
+        }
+        // a multiplier beyond the bound, or a zero or non-finite pivot (its own row's multiplier is 1)
+        if (!(big0 * fabs(p0) <= T(kLaneMaxGrowth)) || !(big1 * fabs(p1) <= T(kLaneMaxGrowth))) bad = 1;
+        if (!(fabs(pa) > T(0)) || !(fabs(e) > T(0))) bad = 1;
+        if (pc == b || pc == b + 1) {  // the pivot columns become the inverse's
+          q1[tc] = pc == b ? -l * p1 : p1;
+          q0[tc] = Num<T>::mul_sub(w, q1[tc], pc == b ? p0 : T(0));
+#pragma unroll
+          for (int a = 0; a < TR; ++a) t[a][tc] = T(0);
+        }
+#pragma unroll
+        for (int a = 0; a < TR; ++a)
+#pragma unroll
+          for (int c = 0; c < TC; ++c)
+            t[a][c] = Num<T>::mul_sub(l1[a], q1[c], Num<T>::mul_sub(l0[a], q0[c], t[a][c]));
+        if (pr == r0 + b) {
+#pragma unroll
+          for (int c = 0; c < TC; ++c) t[ta][c] = q0[c];
+        }
+        if (pr == r0 + b + 1) {
+#pragma unroll
+          for (int c = 0; c < TC; ++c) t[ta][c] = q1[c];
+        }
+        if (b + 2 < GC) {
+          const Shared<T> n{pub.at + (((k >> 1) + 1) & 1) * 4 * kStep};
+          const int rr = pr - (r0 + b + 2), cc = pc - (b + 2);
+          if (rr == 0 || rr == 1)
+#pragma unroll
+            for (int c = 0; c < TC; ++c) n.store((rr * N + pc + GC * c) * S, t[ta][c]);
+          if (cc == 0 || cc == 1)
+#pragma unroll
+            for (int a = 0; a < TR; ++a) n.store(((2 + cc) * N + pr + GR * a) * S, t[a][tc]);
+          __syncthreads();
+        }
+      }
+      if (blk + 1 < TR * F) {  // the next pivots open the next tile row or column (GC / 2 is even: buffer 0)
+        const int na = (blk + 1) / F, rr = pr - GC * ((blk + 1) % F);
+        if (rr == 0 || rr == 1)
+#pragma unroll
+          for (int c = 0; c < TC; ++c) pub.store((rr * N + pc + GC * c) * S, t[na][c]);
+        if (pc < 2)
+#pragma unroll
+          for (int a = 0; a < TR; ++a) pub.store(((2 + pc) * N + pr + GR * a) * S, t[a][blk + 1]);
+        __syncthreads();
+      }
+    }
+#pragma unroll
+    for (int a = 0; a < TR; ++a)
+#pragma unroll
+      for (int c = 0; c < TC; ++c) A.store(((pr + GR * a) * ST + pc + GC * c) * S, t[a][c]);
+    __syncthreads();
+  }
+
+  // The tail of the factorization, where there is one.
+  __device__ __forceinline__ void tail() {
+    if constexpr (kRefine) {
+      switch (K.p.n_t / lane_grid_rows(P)) {
+        case 0: break;
+        case lane_tile(P, 0): invert_tail<lane_tile(P, 0)>(); break;
+        case lane_tile(P, 1): invert_tail<lane_tile(P, 1)>(); break;
+        case lane_tile(P, 2): invert_tail<lane_tile(P, 2)>(); break;
+        default: invert_tail<lane_tile(P, 3)>(); break;
+      }
+    }
+  }
+
+  // The tail rows of the vector section times the tail's inverse.
+  __device__ __forceinline__ void apply_tail() {
+    if constexpr (kRefine) {
+      const int n = K.p.n_t;
+      if (n == 0) return;
+      const Shared<T> z{lus().at + (K.p.vec + K.p.ms) * S * static_cast<uint32_t>(sizeof(T))};
+      constexpr int NR = (lane_tile(P, 3) * lane_grid_rows(P) + P - 1) / P;
+      T out[NR];
+#pragma unroll
+      for (int a = 0; a < NR; ++a) {
+        const int i = slot + P * a;
+        T s0 = T(0), s1 = T(0);
+        if (i < n) {
+          const Shared<T> row{lus().at + (K.p.tail + i * lane_tail_stride(P, n)) * S * static_cast<uint32_t>(sizeof(T))};
+#pragma unroll 4
+          for (int j = 0; j < n; j += 2) {
+            const T a0 = row.load(j * S), z0 = z.load(j * S), a1 = row.load((j + 1) * S), z1 = z.load((j + 1) * S);
+            s0 = Num<T>::mul_sub(a0, -z0, s0);
+            s1 = Num<T>::mul_sub(a1, -z1, s1);
+          }
+        }
+        out[a] = s0 + s1;
+      }
+      __syncthreads();
+#pragma unroll
+      for (int a = 0; a < NR; ++a)
+        if (slot + P * a < n) z.store((slot + P * a) * S, out[a]);
+      __syncthreads();
+    }
+  }
+
+  // The assembled matrix's factors.
+  __device__ __forceinline__ void factorize() {
+    run_lu<kPair>(LS_FACTOR, chunk_space(K.s.q, K.s.ctl));  // q is free
+    tail();
+  }
+
+  // z = (I - c J)^-1 z on the vector section; q is free.
+  __device__ __forceinline__ void solve() {
+    run_lu<1>(LS_FORWARD, chunk_space(K.s.q, K.s.ctl));
+    apply_tail();
+    run_lu<1>(LS_BACKWARD, chunk_space(K.s.q, K.s.ctl));
+  }
+
+  // Rates of progress into q: q = keff x[a] x[b] x[c] (x[m] = 1).
+  __device__ __forceinline__ void rates(const double (&keff)[NRS]) const {
+    const Shared<double> x = xsh(), q = qsh();
+    int n_rounds;
+    const uint4* p = packets(LS_REACTIONS, n_rounds);
+#pragma unroll
+    for (int k = 0; k < NRS; ++k) {
+      if (k >= K.p.nrs) break;
+      const uint4 f = p[k * SPW];
+      if (k * P + slot < K.a.mech.L.R) {
+        double v = keff[k] * x.load((f.x & 0xffffu) * S);
+        if ((f.y >> 16) > 1) v *= x.load((f.x >> 16) * S);
+        if ((f.y >> 16) > 2) v *= x.load((f.y & 0xffffu) * S);
+        q.store(f.w * S, v);
+      }
+    }
+  }
+
+  // dq/dx . v into q.
+  __device__ __forceinline__ void rate_derivatives(const double (&keff)[NRS]) const {
+    const Shared<double> x = xsh(), q = qsh(), v{base() + K.s.v + s * 8u};
+    int n_rounds;
+    const uint4* p = packets(LS_REACTIONS, n_rounds);
+#pragma unroll
+    for (int k = 0; k < NRS; ++k) {
+      if (k >= K.p.nrs) break;
+      const uint4 f = p[k * SPW];
+      if (k * P + slot < K.a.mech.L.R) {
+        const int a = (f.x & 0xffffu) * S, b = (f.x >> 16) * S, c = (f.y & 0xffffu) * S, n = f.y >> 16;
+        double d = n > 0 ? v.load(a) : 0.0;
+        if (n >= 2) {
+          const double xa = x.load(a), xb = x.load(b);
+          d = fma(d, xb, xa * v.load(b));
+          if (n > 2) d = fma(d, x.load(c), xa * xb * v.load(c));
+        }
+        q.store(f.w * S, keff[k] * d);
+      }
+    }
+  }
+
+  // out[k] = sum of nu q over the slot's species.
+  __device__ __forceinline__ void net(double (&out)[NPS]) const {
+    const Shared<double> q = qsh();
+    int n_rounds, e = 0;
+    const uint4* p = packets(LS_NET, n_rounds);
+    const int4 ends = reinterpret_cast<const int4*>(sm + K.s.prog + LS_COUNT * W * sizeof(int2))[warp];
+    const int end[kLaneSegments] = {ends.x, ends.y, ends.z, ends.w};
+#pragma unroll
+    for (int k = 0; k < NPS; ++k) {
+      double a0 = 0.0, a1 = 0.0;
+#pragma unroll 2
+      for (; e < end[k]; e += 2) {
+        const uint4 u = p[0], w = p[SPW];
+        p += 2 * SPW;
+        a0 = fma(__hiloint2double(static_cast<int>(u.w), static_cast<int>(u.z)), q.load(u.x * S), a0);
+        a1 = fma(__hiloint2double(static_cast<int>(w.w), static_cast<int>(w.z)), q.load(w.x * S), a1);
+      }
+      out[k] = a0 + a1;
+    }
+  }
+
+  // dq/dx per factor slot into d, from the iterate in T precision.
+  __device__ __forceinline__ void factor_slots(const T (&kt)[NRS]) const {
+    const Shared<T> x{base() + (kRefine ? K.s.v : K.s.x) + s * static_cast<uint32_t>(sizeof(T))};
+    const Shared<T> d{base() + K.s.q + s * static_cast<uint32_t>(sizeof(T))};
+    int n_rounds;
+    const uint4* p = packets(LS_REACTIONS, n_rounds);
+#pragma unroll
+    for (int k = 0; k < NRS; ++k) {
+      if (k >= K.p.nrs) break;
+      const uint4 f = p[k * SPW];
+      if (k * P + slot < K.a.mech.L.R) {
+        const int n = f.y >> 16;
+        const uint32_t o = f.z * S;
+        if (n == 1) {
+          d.store(o, kt[k]);
+        } else if (n > 1) {
+          const T a = x.load((f.x & 0xffffu) * S), b = x.load((f.x >> 16) * S);
+          if (n == 2) {
+            d.store(o, kt[k] * b);
+            d.store(o + S, kt[k] * a);
+          } else {
+            const T c = x.load((f.y & 0xffffu) * S);
+            d.store(o, kt[k] * b * c);
+            d.store(o + S, kt[k] * a * c);
+            d.store(o + 2 * S, kt[k] * a * b);
+          }
+        }
+      }
+    }
+  }
+
+  // Entries of I - coef J.
+  __device__ __forceinline__ void matrix(T coef) const {
+    const Shared<T> A = lus(), d{base() + K.s.q + s * static_cast<uint32_t>(sizeof(T))};
+    T acc = T(0);
+    // x in T precision (in v's place) has been read; FP64 has no such section
+    int n;
+    Reader r = open<2>(LS_MATRIX, kRefine ? chunk_space(K.s.v, K.s.q) : make_uint2(K.s.stage, K.s.stage_bytes), n);
+#pragma unroll 1
+    for (; n > 0; n -= 2) {
+      const uint4 w0 = r.a, w1 = r.b;
+      // both packets' operands first
+      T nu[2], dv[2], nv[2], ev[2];  // FP32 packets hold two contributions, FP64 packets one
+      if constexpr (sizeof(T) == 4) {
+        nu[0] = __uint_as_float(w0.z), nv[0] = __uint_as_float(w0.w);
+        nu[1] = __uint_as_float(w1.z), nv[1] = __uint_as_float(w1.w);
+        dv[0] = d.load((w0.y & 0xffffu) * S), ev[0] = d.load((w0.y >> 16) * S);
+        dv[1] = d.load((w1.y & 0xffffu) * S), ev[1] = d.load((w1.y >> 16) * S);
+      } else {
+        nu[0] = __hiloint2double(static_cast<int>(w0.w), static_cast<int>(w0.z));
+        nu[1] = __hiloint2double(static_cast<int>(w1.w), static_cast<int>(w1.z));
+        dv[0] = d.load(w0.y * S);
+        dv[1] = d.load(w1.y * S);
+      }
+      advance<2>(r);
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        const uint32_t h = i ? w1.x : w0.x;
+        acc = Num<T>::mul_sub(nu[i], -dv[i], (h & LM_START) ? T(0) : acc);
+        if (sizeof(T) == 4) acc = Num<T>::mul_sub(nv[i], -ev[i], acc);
+        if (h & LM_END) A.store((h & 0x7fffu) * S, Num<T>::mul_sub(coef, acc, (h & LM_DIAG) ? T(1) : T(0)));
+      }
+    }
+  }
+
+  // 0.9 e^(-1/3) clamped to [0.2, 2]: a single-precision start and two Newton-Raphson passes of
+  // r <- r + r (1 - e r^3) / 3, each of which squares the relative error (1e-6 at the start). The control
+  // warp waits for this chain once per step; outside [0.05, 200] the clamp decides alone.
+  static __device__ __forceinline__ double step_factor(double e) {
+    if (!(e > 0.05)) return 2.0;
+    if (e > 200.0) return 0.2;
+    double r = static_cast<double>(exp2f(-log2f(static_cast<float>(e)) * (1.f / 3.f)));
+#pragma unroll
+    for (int i = 0; i < 2; ++i) r = fma(r * (1.0 / 3.0), fma(-e * r, r * r, 1.0), r);
+    return fmax(0.2, fmin(2.0, 0.9 * r));
+  }
+
+  // The next try of sample i's step: clamps the step size, or ends the sample.
+  __device__ __forceinline__ int begin_try(int i, int code) {
+    const double d = 0.5 * (2.0 - sqrt(2.0));
+    double dt = fmin(fmax(cd(D_DT, i), cd(D_DTMIN, i)), cd(D_DTMAX, i));
+    const double left = cd(D_TEND, i) - cd(D_T, i);
+    const bool last = dt >= left;
+    if (last) dt = left;
+    cd(D_DT, i) = dt;
+    ci(I_LAST, i) = last ? 1 : 0;
+    ci(I_STAGE, i) = 0;
+    ci(I_NEWT, i) = 0;
+    if (!(dt > 0.0)) {
+      ci(I_STATUS, i) = TCHEM_GB_SAMPLE_DT_UNDERFLOW;
+      return C_DONE;
+    }
+    cd(D_COEF, i) = d * dt;
+    return code;
+  }
+  // The next step of sample i, or its end.
+  __device__ __forceinline__ int begin_step(int i, int code) {
+    if (!(ci(I_ITER, i) < ci(I_MAXITER, i) && cd(D_T, i) < cd(D_TEND, i))) return C_DONE;
+    ci(I_TRY, i) = 0;
+    return begin_try(i, code);
+  }
+
+  // A slot's value summed (or its maximum taken) over the warp's slots, in every lane.
+  template <bool MAX>
+  static __device__ __forceinline__ double over_warp(double v) {
+#pragma unroll
+    for (int o = S; o < 32; o <<= 1) {
+      const double w = __shfl_xor_sync(kFullMask, v, o);
+      v = MAX ? max_nonneg(v, w) : v + w;
+    }
+    return v;
+  }
+  // The larger of two non-negative numbers, which order as their bit patterns: integer compares instead
+  // of FP64 ones.
+  static __device__ __forceinline__ double max_nonneg(double a, double b) {
+    return __longlong_as_double(max(__double_as_longlong(a), __double_as_longlong(b)));
+  }
+
+  // Sum (or maximum) over the warps of the W partial values at q[(base + warp) * S], by one warp; the
+  // lane's sample is s.
+  template <bool MAX>
+  __device__ __forceinline__ double reduce(int base) const {
+    const double* q = qs();
+    double v = 0.0;
+#pragma unroll
+    for (int k = sl; k < W; k += SPW) {
+      const double w = q[(base + k) * S];
+      v = MAX ? max_nonneg(v, w) : v + w;
+    }
+    return over_warp<MAX>(v);
+  }
+
+  __device__ void run() {
+    const AdvanceParams& A = K.a;
+    const MechLayout& L = A.mech.L;
+    const int mm = m();
+    const double gamma = 2.0 - sqrt(2.0);
+    const double cg = 1.0 / (gamma * (2.0 - gamma));
+    const double cn = (1.0 - gamma) * (1.0 - gamma) / (gamma * (2.0 - gamma));
+    const double kappa = (-3.0 * gamma * gamma + 4.0 * gamma - 2.0) / (12.0 * (2.0 - gamma));
+    const double e0 = 1.0 / gamma, e1 = -1.0 / (gamma * (1.0 - gamma)), e2 = 1.0 / (1.0 - gamma);
+    const int n_items = A.n_items_dev ? *A.n_items_dev : A.n_items;
+    const bool control = warp == 0;
+    const int zbase = K.p.vec * S;  // the vector section of lu
+
+    // the slot's species: positions (mm: none) and, in the upper half, species numbers
+    int sps[NPS];
+#pragma unroll
+    for (int k = 0; k < NPS; ++k) sps[k] = k < K.p.nps ? __ldg(K.p.species + k * P + slot) : mm;
+    auto pos = [&](int k) { return sps[k] & 0xffff; };
+    auto species = [&](int k) { return sps[k] >> 16; };
+    auto has = [&](int k) { return (sps[k] & 0xffff) < mm; };
+    // the iterate itself is x
+    double yn[NPS], fn[NPS], fg[NPS], rv[NPS], keff[NRS];
+    T kt[NRS];
+#pragma unroll
+    for (int k = 0; k < NPS; ++k) {
+      yn[k] = fn[k] = fg[k] = rv[k] = 0.0;
+      if (has(k)) xs()[pos(k) * S] = 0.0;
+    }
+#pragma unroll
+    for (int k = 0; k < NRS; ++k) {
+      keff[k] = 0.0;
+      kt[k] = T(0);
+    }
+    // the resident streams and the small tables
+    for (int id = 0; id < LS_COUNT; ++id)
+      if (K.s.stream[id])
+        for (int i = threadIdx.x; i < K.p.packet_count[id]; i += NT)
+          reinterpret_cast<uint4*>(sm + K.s.stream[id])[i] = __ldg(K.p.packets[id] + i);
+    for (int i = threadIdx.x; i < K.p.table_bytes / 16; i += NT)
+      reinterpret_cast<uint4*>(sm + K.s.prog)[i] = __ldg(K.p.table + i);
+    if (s == 0)
+#pragma unroll
+      for (int k = 0; k < NPS; ++k)
+        if (has(k))
+          reinterpret_cast<double2*>(sm + K.s.tol)[pos(k)] = make_double2(A.tol_time[2 * species(k)], A.tol_time[2 * species(k) + 1]);
+    if (slot == 0) {
+      xs()[mm * S] = 1.0;
+      lu()[K.p.zero * S] = T(0);
+      lu()[K.p.ms * S] = T(1);
+      for (int k = K.p.vec + mm; k < K.p.n_entries; ++k) lu()[k * S] = T(0);  // tail rows beyond the species
+    }
+    if (control && sl == 0) {
+      ci(I_CODE, s) = C_IDLE;
+      ci(I_SMP, s) = -1;
+      cd(D_COEF, s) = 0.0;
+      ci(I_BAD, s) = 0;
+    }
+    if (threadIdx.x == 0) flag(0) = 1;  // some lane wants a sample
+    const double* srcp = K.p.emis;
+    int dead = 0;  // control lanes: the queue gave out
+    __syncthreads();
+
+    while (true) {
+      // ---- new samples ----
+      if (flag(0)) {
+        bool fresh = false;
+        if (control && sl == 0 && ci(I_CODE, s) == C_IDLE && !dead) {
+          int smp = -1;
+          while (true) {
+            const int item = atomicAdd(A.queue, 1);
+            if (item >= n_items) {
+              dead = 1;
+              break;
+            }
+            const int c = A.items ? A.items[item] : item;
+            const tchem_gb_tadv ta = A.tadv[c];
+            if (A.t_out[c] >= ta.tend) {
+              A.status[c] = TCHEM_GB_SAMPLE_SKIPPED;
+              if (A.stats) A.stats[c] = tchem_gb_sample_stats{};
+              continue;
+            }
+            const int gm = A.mech_of_sample ? A.mech_of_sample[c] : 0;
+            const int sm_slot = (gm >= 0 && gm < kMaxMechs) ? A.slot_of_mech[gm] : -1;
+            if (sm_slot < 0) {
+              A.status[c] = TCHEM_GB_SAMPLE_BAD_MECH;
+              continue;
+            }
+            if (ta.dt < 0.0 || ta.jacobian_interval > 1 || ta.max_num_newton_iterations < 1) {
+              A.status[c] = kStatusRedo;  // cases the general kernel handles
+              atomicAdd(K.redo_count, 1);
+              continue;
+            }
+            smp = c;
+            cd(D_T, s) = ta.tbeg;
+            cd(D_DT, s) = ta.dt;
+            cd(D_TEND, s) = ta.tend;
+            cd(D_DTMIN, s) = ta.dtmin;
+            cd(D_DTMAX, s) = ta.dtmax;
+            ci(I_MAXITER, s) = ta.num_time_iterations_per_interval;
+            ci(I_MAXNEWT, s) = ta.max_num_newton_iterations;
+            ci(I_ITER, s) = 0;
+            ci(I_STEPS, s) = ci(I_REJ, s) = ci(I_NFAIL, s) = ci(I_NITS, s) = ci(I_NOK0, s) = ci(I_NATT, s) = 0;
+            ci(I_STATUS, s) = TCHEM_GB_SAMPLE_OK;
+            ci(I_SLOT, s) = sm_slot;
+            ci(I_ACC, s) = 0;
+            break;
+          }
+          ci(I_SMP, s) = smp;
+          fresh = smp >= 0;
+          if (fresh) ci(I_CODE, s) = C_FRESH;
+        }
+        __syncthreads();
+        // rate constants of the new samples: all threads over (sample, reaction), through q
+        bool any = false;
+        for (int c = 0; c < S; ++c) {
+          if (ci(I_CODE, c) != C_FRESH) continue;
+          any = true;
+          const int smp = ci(I_SMP, c);
+          const double* row = A.state + static_cast<size_t>(smp) * A.state_dim;
+          const double p = row[1], Tk = row[2], t_1 = 1.0 / Tk, conv = A.mech.conv_ppm * p * t_1;
+          const double* rp = A.keff_in ? nullptr : A.rate_param[ci(I_SLOT, c)];
+          double* q = reinterpret_cast<double*>(sm + K.s.q) + c;
+          for (int r = threadIdx.x; r < L.R; r += NT) {
+            double k;
+            if (A.keff_in) {
+              k = A.keff_in[static_cast<size_t>(smp) * L.R + r];
+            } else {
+              k = rate_constant(A.mech.rate_type[r], rp + 8 * r, A.mech.conv_exp[r], Tk, t_1, p, conv);
+              for (int e = A.mech.cf_ptr[r]; e < A.mech.cf_ptr[r + 1]; ++e) k *= row[3 + mm + A.mech.cf_idx[e]];
+            }
+            if (A.k_scale) k *= A.k_scale[r];
+            q[r * S] = k;
+          }
+        }
+        __syncthreads();
+        if (!any) {
+          bool idle = true;
+          for (int c = 0; c < S; ++c) idle = idle && ci(I_CODE, c) == C_IDLE;
+          if (idle) break;  // every lane is idle and the queue is empty
+        }
+        if (ci(I_CODE, s) == C_FRESH) {
+          const int smp = ci(I_SMP, s);
+          const double* row = A.state + static_cast<size_t>(smp) * A.state_dim;
+          int n_rounds;
+          const uint4* rx = packets(LS_REACTIONS, n_rounds);
+#pragma unroll
+          for (int k = 0; k < NRS; ++k)
+            if (k < K.p.nrs && k * P + slot < L.R) {
+              keff[k] = qs()[rx[k * SPW].w * S];
+              kt[k] = static_cast<T>(keff[k]);
+            }
+#pragma unroll
+          for (int k = 0; k < NPS; ++k) {
+            yn[k] = has(k) ? row[3 + species(k)] : 0.0;
+            if (has(k)) xs()[pos(k) * S] = yn[k];
+            fn[k] = fg[k] = rv[k] = 0.0;
+          }
+          if (A.keff_in) srcp = A.src_in + smp * A.src_stride;
+        }
+        __syncthreads();
+        if (fresh) ci(I_CODE, s) = begin_step(s, C_FRESH);
+        __syncthreads();
+      }
+
+      // ---- right-hand side at the iterate ----
+      int code = ci(I_CODE, s);
+      double coef = cd(D_COEF, s);
+      if (threadIdx.x == 0) flag(0) = 0;
+      if (code == C_RETRY) {
+#pragma unroll
+        for (int k = 0; k < NPS; ++k)
+          if (has(k)) xs()[pos(k) * S] = yn[k];
+      }
+      if (slot == 0) qs()[L.R * S] = 0.0;
+      double src[NPS];
+#pragma unroll
+      for (int k = 0; k < NPS; ++k) src[k] = has(k) ? __ldg(srcp + species(k)) : 0.0;
+      __syncthreads();
+      rates(keff);
+      const int step_pending = __syncthreads_or(code == C_STEP || code == C_DONE);
+      double f[NPS];
+      net(f);
+#pragma unroll
+      for (int k = 0; k < NPS; ++k)
+        if (has(k)) f[k] += src[k];
+
+      // ---- error test of the samples whose second stage converged ----
+      if (step_pending) {
+        __syncthreads();  // q is read
+        const double dt = cd(D_DT, s);
+#pragma unroll
+        for (int k = 0; k < NPS; ++k)
+          if (has(k)) {
+            const double est = code == C_STEP ? 2.0 * kappa * dt * (e0 * fn[k] + e1 * fg[k] + e2 * f[k]) : 0.0;
+            lu()[zbase + pos(k) * S] = static_cast<T>(est);
+          }
+        __syncthreads();
+        solve();
+        // the largest |est| / weight of the slot's species: the quotients are compared by cross products
+        // (one division; as fmax does, a NaN quotient loses every comparison)
+        double num = 0.0, den = 1.0;
+        if (code == C_STEP) {
+#pragma unroll
+          for (int k = 0; k < NPS; ++k)
+            if (has(k)) {
+              const double est = fabs(static_cast<double>(lu()[zbase + pos(k) * S]));
+              const double2 tol = reinterpret_cast<const double2*>(sm + K.s.tol)[pos(k)];
+              const double wgt = tol.x + tol.y * fmax(fabs(yn[k]), fabs(xs()[pos(k) * S]));
+              if (est * den > num * wgt) {
+                num = est;
+                den = wgt;
+              }
+            }
+        }
+        num = over_warp<true>(num > 0.0 ? num / den : 0.0);
+        if (sl == 0) qs()[warp * S] = num;
+        __syncthreads();
+        if (control) {
+          const double e = reduce<true>(0);
+          if (sl == 0 && code == C_STEP) {
+            ++ci(I_NATT, s);
+            int next;
+            const double h = cd(D_DT, s);
+            if (!isfinite(e)) {
+              ci(I_STATUS, s) = TCHEM_GB_SAMPLE_NONFINITE;
+              ci(I_ACC, s) = 0;
+              next = C_DONE;
+            } else if ((e <= 1.0 || h <= cd(D_DTMIN, s)) && A.tape_dt && ci(I_STEPS, s) >= A.tape_cap) {
+              ci(I_STATUS, s) = TCHEM_GB_SAMPLE_TAPE_FULL;
+              ci(I_ACC, s) = 0;
+              next = C_DONE;
+            } else if (e <= 1.0 || h <= cd(D_DTMIN, s)) {
+              const double t = ci(I_LAST, s) ? cd(D_TEND, s) : cd(D_T, s) + h;
+              const double fac = step_factor(e);
+              double hn = fmin(h * fac, cd(D_DTMAX, s));
+              if (t + hn > cd(D_TEND, s)) hn = cd(D_TEND, s) - t;
+              if (A.tape_dt) A.tape_dt[static_cast<size_t>(ci(I_SMP, s)) * A.tape_cap + ci(I_STEPS, s)] = h;
+              cd(D_T, s) = t;
+              cd(D_DT, s) = hn;
+              ++ci(I_STEPS, s);
+              ++ci(I_ITER, s);
+              ci(I_ACC, s) = 1;
+              next = begin_step(s, C_ACCEPT);
+            } else {
+              ++ci(I_REJ, s);
+              ++ci(I_ITER, s);
+              ci(I_ACC, s) = 0;
+              cd(D_DT, s) = h * step_factor(e);  // e > 1: below 0.9
+              next = begin_step(s, C_REJECT);
+            }
+            ci(I_CODE, s) = next;
+          }
+        }
+        __syncthreads();
+        if (A.tape_dt && code == C_STEP && ci(I_ACC, s)) {
+          // checkpoint: the state at the start of the step just accepted
+          const int n = ci(I_STEPS, s) - 1;
+          if (n % kTapeSegment == 0) {
+            double* ck = A.tape_ckpt + (static_cast<size_t>(ci(I_SMP, s)) * (A.tape_cap / kTapeSegment + 1) + n / kTapeSegment) * mm;
+#pragma unroll
+            for (int k = 0; k < NPS; ++k)
+              if (has(k)) ck[species(k)] = yn[k];
+          }
+        }
+        code = ci(I_CODE, s);
+        coef = cd(D_COEF, s);
+        if (code == C_DONE) {
+          const int smp = ci(I_SMP, s), status = ci(I_STATUS, s);
+          if (status == kStatusRedo) {
+            if (slot == 0) {
+              A.status[smp] = kStatusRedo;
+              atomicAdd(K.redo_count, 1);
+            }
+          } else {
+            const bool at_y = ci(I_ACC, s) != 0;  // else y_n: the last attempt was rejected, or no step was taken
+            const double* row = A.state + static_cast<size_t>(smp) * A.state_dim;
+            double* out = A.state_out + static_cast<size_t>(smp) * A.state_dim;
+            for (int i = slot; i < A.state_dim - 3 - mm; i += P) out[3 + mm + i] = row[3 + mm + i];
+#pragma unroll
+            for (int k = 0; k < NPS; ++k)
+              if (has(k)) out[3 + species(k)] = status != TCHEM_GB_SAMPLE_OK ? 0.0 : (at_y ? xs()[pos(k) * S] : yn[k]);
+            if (slot == 0) {
+              const double rho = row[0], p = row[1], Tk = row[2];
+              out[0] = rho;
+              out[1] = p;
+              out[2] = Tk;
+              A.t_out[smp] = status == TCHEM_GB_SAMPLE_OK ? cd(D_T, s) : cd(D_TEND, s);
+              A.dt_out[smp] = status == TCHEM_GB_SAMPLE_OK ? cd(D_DT, s) : -1.0;
+              A.status[smp] = status;
+              if (A.tape_nsteps) A.tape_nsteps[smp] = ci(I_STEPS, s);
+              if (A.stats) {
+                tchem_gb_sample_stats st;
+                st.n_steps = ci(I_STEPS, s);
+                st.n_rejected = ci(I_REJ, s);
+                st.n_newton_fail = ci(I_NFAIL, s);
+                st.n_newton_iter = ci(I_NITS, s);
+                st.n_lu = st.n_jac = ci(I_NITS, s);
+                // as the algorithm counts them: f(y_0), one per iteration (and one Jacobian-vector
+                // product per refinement), f(y_gamma) and f(y_{n+1})
+                st.n_solve = (kRefine ? 2 : 1) * ci(I_NITS, s) + ci(I_NATT, s);
+                st.n_rhs = 1 + (kRefine ? 2 : 1) * ci(I_NITS, s) + ci(I_NOK0, s) + ci(I_NATT, s);
+                A.stats[smp] = st;
+              }
+            }
+          }
+        }
+        if (code == C_ACCEPT) {
+#pragma unroll
+          for (int k = 0; k < NPS; ++k)
+            if (has(k)) {
+              yn[k] = xs()[pos(k) * S];
+              fn[k] = f[k];
+            }
+        } else if (code == C_REJECT) {
+#pragma unroll
+          for (int k = 0; k < NPS; ++k) {
+            f[k] = fn[k];
+            if (has(k)) xs()[pos(k) * S] = yn[k];
+          }
+        }
+        __syncthreads();  // outputs written before the lane is given away
+        if (control && sl == 0 && code == C_DONE) {
+          ci(I_CODE, s) = C_IDLE;
+          ci(I_SMP, s) = -1;
+          cd(D_COEF, s) = 0.0;
+          flag(0) = 1;
+        }
+      }
+
+      // ---- where the stage starts ----
+      if (code == C_STAGE) {
+#pragma unroll
+        for (int k = 0; k < NPS; ++k)
+          if (has(k)) {
+            fg[k] = f[k];
+            rv[k] = cg * xs()[pos(k) * S] - cn * yn[k];
+          }
+      } else if (code != C_ITER) {
+        if (code == C_FRESH) {
+#pragma unroll
+          for (int k = 0; k < NPS; ++k) fn[k] = f[k];
+        }
+#pragma unroll
+        for (int k = 0; k < NPS; ++k)
+          if (has(k)) rv[k] = yn[k] + coef * fn[k];
+      }
+
+      double g[NPS], dx[NPS];
+#pragma unroll
+      for (int k = 0; k < NPS; ++k) {
+        g[k] = 0.0;
+        if (has(k)) {
+          const double y = xs()[pos(k) * S];
+          g[k] = -((y - coef * f[k]) - rv[k]);
+          lu()[zbase + pos(k) * S] = static_cast<T>(g[k]);
+          if (kRefine) xt()[pos(k) * S] = static_cast<T>(y);
+        }
+      }
+      bad = 0;
+      {
+        // zero the pattern behind the pivots and the one entry (the matrix stream writes every pivot)
+        T* z = reinterpret_cast<T*>(sm + K.s.lu) + (K.p.ms + 1) * S;
+        const int n = (K.p.zero - K.p.ms - 1) * S;
+        if constexpr (S * sizeof(T) >= 16) {
+          for (int i = threadIdx.x; i < n * static_cast<int>(sizeof(T)) / 16; i += NT)
+            reinterpret_cast<uint4*>(z)[i] = make_uint4(0u, 0u, 0u, 0u);
+        } else {
+          for (int i = threadIdx.x; i < n; i += NT) z[i] = T(0);
+        }
+      }
+      __syncthreads();
+      factor_slots(kt);
+      if (slot == 0) ds()[L.NF * S] = T(0);
+      __syncthreads();
+      matrix(static_cast<T>(coef));
+      if constexpr (kRefine) {
+        // g waits in v, which matrix() no longer needs as chunk space, for the refinement
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < NPS; ++k)
+          if (has(k)) vs()[pos(k) * S] = g[k];
+      }
+      __syncthreads();
+      factorize();
+      if (bad) ci(I_BAD, s) = 1;
+      solve();
+#pragma unroll
+      for (int k = 0; k < NPS; ++k) dx[k] = has(k) ? static_cast<double>(lu()[zbase + pos(k) * S]) : 0.0;
+      if constexpr (kRefine) {
+        // FP64 residual of (I - c J) dx = g, correction through the FP32 factors
+#pragma unroll
+        for (int k = 0; k < NPS; ++k)
+          if (has(k)) {
+            g[k] = vs()[pos(k) * S];
+            vs()[pos(k) * S] = dx[k];
+          }
+        if (slot == 0) qs()[L.R * S] = 0.0;
+        __syncthreads();
+        rate_derivatives(keff);
+        __syncthreads();
+        double jd[NPS];
+        net(jd);
+#pragma unroll
+        for (int k = 0; k < NPS; ++k)
+          if (has(k)) lu()[zbase + pos(k) * S] = static_cast<T>(g[k] - (dx[k] - coef * jd[k]));
+        __syncthreads();
+        solve();
+#pragma unroll
+        for (int k = 0; k < NPS; ++k)
+          if (has(k)) dx[k] += static_cast<double>(lu()[zbase + pos(k) * S]);
+      }
+      double sdx = 0.0, sy = 0.0;
+#pragma unroll
+      for (int k = 0; k < NPS; ++k)
+        if (has(k)) {
+          const double y = xs()[pos(k) * S] + dx[k];
+          xs()[pos(k) * S] = y;
+          sdx += dx[k] * dx[k];
+          sy += y * y;
+        }
+      sdx = over_warp<false>(sdx);
+      sy = over_warp<false>(sy);
+      if (sl == 0) {
+        qs()[warp * S] = sdx;
+        qs()[(W + warp) * S] = sy;
+      }
+      __syncthreads();
+      if (warp == 1) {  // ||y|| beside the control warp's ||dx||
+        const double v = sqrt(reduce<false>(W));
+        if (sl == 0) qs()[2 * W * S] = v;
+        asm volatile("bar.arrive 1, 64;" ::: "memory");
+      }
+      if (control) {
+        const double ndx = sqrt(reduce<false>(0));
+        asm volatile("bar.sync 1, 64;" ::: "memory");
+        const double ny = qs()[2 * W * S];
+        if (sl == 0 && ci(I_SMP, s) >= 0) {
+          int next = C_ITER;
+          ++ci(I_NITS, s);
+          const int it = ++ci(I_NEWT, s);
+          const bool finite = isfinite(ndx) && isfinite(ny);
+          if (ci(I_BAD, s)) {
+            ci(I_BAD, s) = 0;
+            ci(I_STATUS, s) = kStatusRedo;
+            next = C_DONE;
+          } else if (finite && ndx <= A.tol_newton[0] + A.tol_newton[1] * ny) {
+            if (ci(I_STAGE, s) == 0) {
+              ci(I_STAGE, s) = 1;
+              ci(I_NEWT, s) = 0;
+              ++ci(I_NOK0, s);
+              next = C_STAGE;
+            } else {
+              next = C_STEP;
+            }
+          } else if (!finite || it >= ci(I_MAXNEWT, s)) {
+            ++ci(I_NFAIL, s);
+            cd(D_DT, s) *= 0.5;
+            if (++ci(I_TRY, s) < 4) {
+              next = begin_try(s, C_RETRY);
+            } else {
+              ci(I_STATUS, s) = TCHEM_GB_SAMPLE_NEWTON_FAIL;
+              next = C_DONE;
+            }
+          }
+          ci(I_CODE, s) = next;
+        } else if (sl == 0) {
+          ci(I_BAD, s) = 0;
+        }
+      }
+      __syncthreads();
+    }
+  }
+};
+
+}  // namespace lanes
+}  // namespace tchem_gb
+
+namespace tchem_gb {
+namespace lanes {
+
+template <typename T, int S, int W, int CTAS>
+__global__ void __launch_bounds__(32 * W, CTAS) trbdf2_lanes_kernel(const __grid_constant__ LaneParams K) {
+  extern __shared__ __align__(128) unsigned char smem[];
+  constexpr int SPW = 32 / S;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  Kernel<T, S, W> k{K, smem, lane % S, lane / S, warp * SPW + lane / S, warp, 0};
+  k.run();
+}
+
+}  // namespace lanes
+}  // namespace tchem_gb
+
+#define TCHEM_GB_LANE_SHAPE(NAME, T, S, W, C)                                                         \
+  namespace tchem_gb {                                                                              \
+  const void* lane_kernel_##NAME() {                                                                \
+    return reinterpret_cast<const void*>(&lanes::trbdf2_lanes_kernel<T, S, W, C>);                       \
+  }                                                                                                 \
+  cudaError_t launch_lanes_##NAME(const LaneParams& P, int grid, cudaStream_t stream) {              \
+    lanes::trbdf2_lanes_kernel<T, S, W, C><<<grid, 32 * W, P.s.bytes, stream>>>(P);                      \
+    return cudaGetLastError();                                                                      \
+  }                                                                                                 \
+  }

@@ -17,8 +17,6 @@ namespace tchem_gb {
   const void* kernel_##PRE##_##MC##_##RPT();
 TCHEM_GB_DECLARE_SHAPE(mixed, 24, 1)
 TCHEM_GB_DECLARE_SHAPE(mixed, 32, 1)
-TCHEM_GB_DECLARE_SHAPE(mixsp, 64, 2)
-TCHEM_GB_DECLARE_SHAPE(mixsp, 128, 4)
 TCHEM_GB_DECLARE_SHAPE(mixgj, 52, 1_g2)
 TCHEM_GB_DECLARE_SHAPE(mixgj, 64, 1_g2)
 TCHEM_GB_DECLARE_SHAPE(mixgj, 128, 1_g4)
@@ -42,47 +40,40 @@ struct Variant {
   bool simplified;  // the form: TCHEM_GB_FORM_MIXED_SIMPLIFIED (else TCHEM_GB_FORM_MIXED)
   bool gj;          // Gauss-Jordan inverse (else LU)
   bool e3;          // E3SM inputs (per-sample rate constants and source terms)
-  bool sp;          // static-order sparse LU (full Newton; needs the mechanism's LU program)
   const void* kernel;
   cudaError_t (*launch)(const AdvanceParams&, int, int, size_t, cudaStream_t);
 };
 
 // Kernel shapes of each form; a mechanism uses the first in table order with MC >= m and
 // 32 G RPT >= m, among those with the requested threads per sample (32 G; 0: any). The E3SM time
-// advance has its own instantiations (up to 64 species). In the full-Newton form, one warp per
-// sample above 32 species is the static-order sparse LU (needs the mechanism's LU program); it
-// comes after the Gauss-Jordan shapes, which measured faster (51 species: 5,621 against 3,248
-// samples/s; 120 species: 436 against 238), so they are the default without a tuned preference.
+// advance has its own instantiations (up to 64 species).
 const Variant* variants(int* n) {
   static const Variant v[] = {
-      {24, 1, 1, 12, false, false, false, false, kernel_mixed_24_1(), &launch_mixed_24_1},
-      {32, 1, 1, 12, false, false, false, false, kernel_mixed_32_1(), &launch_mixed_32_1},
-      {52, 1, 2, 16, false, true, false, false, kernel_mixgj_52_1_g2(), &launch_mixgj_52_1_g2},
-      {64, 1, 2, 12, false, true, false, false, kernel_mixgj_64_1_g2(), &launch_mixgj_64_1_g2},
-      {128, 1, 4, 8, false, true, false, false, kernel_mixgj_128_1_g4(), &launch_mixgj_128_1_g4},
-      {64, 2, 1, 16, false, true, false, true, kernel_mixsp_64_2(), &launch_mixsp_64_2},
-      {128, 4, 1, 8, false, true, false, true, kernel_mixsp_128_4(), &launch_mixsp_128_4},
-      {24, 1, 1, 12, true, true, false, false, kernel_simpl_24_1(), &launch_simpl_24_1},
-      {32, 1, 1, 12, true, true, false, false, kernel_simpl_32_1(), &launch_simpl_32_1},
-      {52, 2, 1, 8, true, true, false, false, kernel_simpl_52_2(), &launch_simpl_52_2},
-      {64, 2, 1, 8, true, true, false, false, kernel_simpl_64_2(), &launch_simpl_64_2},
-      {52, 1, 2, 16, true, true, false, false, kernel_simpl_52_1_g2(), &launch_simpl_52_1_g2},
-      {64, 1, 2, 12, true, true, false, false, kernel_simpl_64_1_g2(), &launch_simpl_64_1_g2},
-      {128, 1, 4, 8, true, true, false, false, kernel_simpl_128_1_g4(), &launch_simpl_128_1_g4},
-      {64, 2, 1, 8, false, false, true, false, kernel_e3mixed_64_2(), &launch_e3mixed_64_2},
-      {64, 2, 1, 8, true, true, true, false, kernel_e3simpl_64_2(), &launch_e3simpl_64_2},
-      {64, 1, 2, 12, true, true, true, false, kernel_e3simpl_64_1_g2(), &launch_e3simpl_64_1_g2},
+      {24, 1, 1, 12, false, false, false, kernel_mixed_24_1(), &launch_mixed_24_1},
+      {32, 1, 1, 12, false, false, false, kernel_mixed_32_1(), &launch_mixed_32_1},
+      {52, 1, 2, 16, false, true, false, kernel_mixgj_52_1_g2(), &launch_mixgj_52_1_g2},
+      {64, 1, 2, 12, false, true, false, kernel_mixgj_64_1_g2(), &launch_mixgj_64_1_g2},
+      {128, 1, 4, 8, false, true, false, kernel_mixgj_128_1_g4(), &launch_mixgj_128_1_g4},
+      {24, 1, 1, 12, true, true, false, kernel_simpl_24_1(), &launch_simpl_24_1},
+      {32, 1, 1, 12, true, true, false, kernel_simpl_32_1(), &launch_simpl_32_1},
+      {52, 2, 1, 8, true, true, false, kernel_simpl_52_2(), &launch_simpl_52_2},
+      {64, 2, 1, 8, true, true, false, kernel_simpl_64_2(), &launch_simpl_64_2},
+      {52, 1, 2, 16, true, true, false, kernel_simpl_52_1_g2(), &launch_simpl_52_1_g2},
+      {64, 1, 2, 12, true, true, false, kernel_simpl_64_1_g2(), &launch_simpl_64_1_g2},
+      {128, 1, 4, 8, true, true, false, kernel_simpl_128_1_g4(), &launch_simpl_128_1_g4},
+      {64, 2, 1, 8, false, false, true, kernel_e3mixed_64_2(), &launch_e3mixed_64_2},
+      {64, 2, 1, 8, true, true, true, kernel_e3simpl_64_2(), &launch_e3simpl_64_2},
+      {64, 1, 2, 12, true, true, true, kernel_e3simpl_64_1_g2(), &launch_e3simpl_64_1_g2},
   };
   *n = static_cast<int>(sizeof(v) / sizeof(v[0]));
   return v;
 }
 
-const Variant* pick(const MechLayout& L, bool simplified, int threads_per_sample, bool e3, int lu_nnz) {
+const Variant* pick(const MechLayout& L, bool simplified, int threads_per_sample, bool e3) {
   int nv = 0;
   const Variant* v = variants(&nv);
   for (int i = 0; i < nv; ++i)
     if (v[i].simplified == simplified && v[i].e3 == e3 && v[i].MC >= L.m && 32 * v[i].G * v[i].RPT >= L.m &&
-        (!v[i].sp || (lu_nnz > 0 && L.off_js_e >= 0)) &&
         (threads_per_sample == 0 || threads_per_sample == 32 * v[i].G))
       return &v[i];
   return nullptr;
@@ -91,10 +82,10 @@ const Variant* pick(const MechLayout& L, bool simplified, int threads_per_sample
 }  // namespace
 
 MixedConfig mixed_config(const MechLayout& L, int threads_per_sample, int sm_count, int max_smem_optin, int nbatch,
-                         bool simplified, bool e3, int lu_nnz) {
+                         bool simplified, bool e3) {
   if (threads_per_sample != 0 && threads_per_sample != 32 && threads_per_sample != 64 && threads_per_sample != 128)
     throw std::domain_error("mixed forms: threads_per_sample must be 0, 32, 64 or 128");
-  const Variant* best = pick(L, simplified, threads_per_sample, e3, lu_nnz);
+  const Variant* best = pick(L, simplified, threads_per_sample, e3);
   if (!best && e3)
     throw std::domain_error("E3SM time advance: the mixed forms have kernel shapes for up to 64 active species "
                             "(32 or 64 threads per sample for the simplified form, 32 for the FP32-LU form); "
@@ -103,9 +94,9 @@ MixedConfig mixed_config(const MechLayout& L, int threads_per_sample, int sm_cou
     throw std::domain_error(simplified ? "simplified form: no kernel shape for this mechanism size and threads_per_sample "
                                          "(up to 64 species with 32 or 64 threads, 128 with 128 threads)"
                                        : "full-Newton FP32 form: no kernel shape for this mechanism size and "
-                                         "threads_per_sample (LU up to 128 species with 32 threads; Gauss-Jordan "
+                                         "threads_per_sample (LU up to 32 species with 32 threads; Gauss-Jordan "
                                          "up to 64 species with 64 threads, 128 with 128 threads)");
-  MixedLayout ml = mixed::make_layout(L, best->MC, best->gj, e3, best->sp ? lu_nnz : 0);
+  MixedLayout ml = mixed::make_layout(L, best->MC, best->gj, e3);
   ml.simplified = simplified ? 1 : (best->gj ? 2 : 0);
   const size_t gbytes = ml.warp_bytes;
   const size_t avail = static_cast<size_t>(max_smem_optin) - 16 - L.blob_bytes;
@@ -129,8 +120,7 @@ MixedConfig mixed_config(const MechLayout& L, int threads_per_sample, int sm_cou
 
 cudaError_t launch_trbdf2_mixed(const AdvanceParams& P, const MechLayout& L, int grid, int warps_per_block,
                                 size_t smem, int threads_per_sample, cudaStream_t stream) {
-  const int lu_nnz = P.mech.lu_prog ? P.mech.lu.nnz : 0;
-  const Variant* best = pick(L, P.ml.simplified == 1, threads_per_sample, P.keff_in != nullptr, lu_nnz);
+  const Variant* best = pick(L, P.ml.simplified == 1, threads_per_sample, P.keff_in != nullptr);
   if (!best) return cudaErrorInvalidValue;
   return best->launch(P, grid, warps_per_block * 32, smem, stream);
 }

@@ -780,6 +780,7 @@ struct Solver {
 
 // One sample per CTA, persistent over the work queue (the outer protocol of the other forms).
 __global__ void __launch_bounds__(kNT, 1) trbdf2_tc_kernel(const __grid_constant__ AdvanceParams P) {
+  if (P.redo_count && *P.redo_count == 0) return;
   extern __shared__ __align__(1024) unsigned char smem[];
   Header* H = reinterpret_cast<Header*>(smem);
   const MechLayout& L = P.mech.L;
@@ -824,6 +825,7 @@ __global__ void __launch_bounds__(kNT, 1) trbdf2_tc_kernel(const __grid_constant
     __syncthreads();
     if (item >= n_items) break;
     const int s = P.items ? P.items[item] : item;
+    if (P.redo_count && P.status[s] != kStatusRedo) continue;  // advanced by the batched kernel
     const tchem_gb_tadv ta = P.tadv[s];
     if (P.t_out[s] >= ta.tend) {
       if (tid == 0) {
