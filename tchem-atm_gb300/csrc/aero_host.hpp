@@ -11,6 +11,15 @@
 namespace tchem_gb {
 
 // The aerosol model's SIMPOL and species tables on one device (one allocation).
+struct LaneTables;
+
+// The batched kernel's instruction streams for one gas mechanism and particle count.
+struct AeroLanes {
+  std::vector<int64_t> signature;  // of the gas mechanism (HostTables::signature)
+  int n_particles = 0;
+  LaneTables* lanes = nullptr;     // null: no shape fits
+};
+
 struct AeroDeviceTables {
   int device = -1;
   const int32_t* sim_idx = nullptr;  // [nSimpol][3], as tchem_gb_aero_view::simpol_index
@@ -18,6 +27,8 @@ struct AeroDeviceTables {
   const double* density = nullptr;   // [nSpec]
   const double* mw = nullptr;        // [nSpec]
   void* allocation = nullptr;
+  // by content, kept until the model is destroyed (launches in flight read them)
+  std::vector<AeroLanes> lanes;
 };
 void destroy_aero_device_tables(AeroDeviceTables* t);  // defined with the device code
 

@@ -50,33 +50,34 @@ struct AeroEval {
   int32_t R;
 };
 
-// Temperature and pressure terms of every SIMPOL entry, NL lanes over entries (lane in [0, NL)).
+// Temperature and pressure terms of one SIMPOL entry (I, P as AeroDev::sim_idx, sim_par).
+__host__ __device__ inline void aero_entry_terms(const int32_t* I, const double* P, double t, double p, double* sc) {
+  const double B1 = P[0], B2 = P[1], B3 = P[2], B4 = P[3], D = P[4], N_star = P[5], MW = P[6];
+  double alpha = 0.1;
+  if (I[2]) {
+    const double n23 = pow(N_star, 2.0 / 3.0);
+    double dh = -10.0 * (N_star - 1.0) + 7.53 * (n23 - 1.0) - 1.0;
+    double ds = -32.0 * (N_star - 1.0) + 9.21 * (n23 - 1.0) - 1.3;
+    dh = dh * 4184.0;
+    ds = ds * 4.184;
+    const double dg = dh - t * ds;
+    alpha = exp(-dg / (kAeroRuniv * t));
+    alpha = alpha / (1.0 + alpha);
+  }
+  double vp = B1 / t + B2 + B3 * t + B4 * log(t);
+  vp = kAeroAtmPa * pow(10.0, vp);
+  sc[0] = alpha;
+  sc[1] = 3.0 * D / sqrt(8.0 * kAeroRuniv * t / (kAeroPi * MW));
+  sc[2] = vp / p / MW * 1.0e6;
+  sc[3] = kAeroRuniv / MW * 1.0e6 * t / p;
+}
+
+// Those of every SIMPOL entry, NL lanes over entries (lane in [0, NL)).
 template <int NL>
 __host__ __device__ inline void aero_setup(const AeroEval& E, int lane, double t, double p) {
   const AeroDev& A = E.A;
-  for (int is = lane; is < A.nS; is += NL) {
-    const int32_t* I = A.sim_idx + 3 * is;
-    const double* P = A.sim_par + 7 * is;
-    const double B1 = P[0], B2 = P[1], B3 = P[2], B4 = P[3], D = P[4], N_star = P[5], MW = P[6];
-    double alpha = 0.1;
-    if (I[2]) {
-      const double n23 = pow(N_star, 2.0 / 3.0);
-      double dh = -10.0 * (N_star - 1.0) + 7.53 * (n23 - 1.0) - 1.0;
-      double ds = -32.0 * (N_star - 1.0) + 9.21 * (n23 - 1.0) - 1.3;
-      dh = dh * 4184.0;
-      ds = ds * 4.184;
-      const double dg = dh - t * ds;
-      alpha = exp(-dg / (kAeroRuniv * t));
-      alpha = alpha / (1.0 + alpha);
-    }
-    double vp = B1 / t + B2 + B3 * t + B4 * log(t);
-    vp = kAeroAtmPa * pow(10.0, vp);
-    double* sc = E.simc + 4 * is;
-    sc[0] = alpha;
-    sc[1] = 3.0 * D / sqrt(8.0 * kAeroRuniv * t / (kAeroPi * MW));
-    sc[2] = vp / p / MW * 1.0e6;
-    sc[3] = kAeroRuniv / MW * 1.0e6 * t / p;
-  }
+  for (int is = lane; is < A.nS; is += NL)
+    aero_entry_terms(A.sim_idx + 3 * is, A.sim_par + 7 * is, t, p, E.simc + 4 * is);
 }
 
 // E.f = RHS at the ODE vector in E.x, NL lanes (a whole warp on the device, NL = 32; one host

@@ -12,12 +12,14 @@
 #include "aero_host.hpp"
 #include "capi_internal.hpp"
 #include "kernels.hpp"
+#include "lane_tables.hpp"
 #include "mech_host.hpp"
 
 namespace tchem_gb {
 
 void destroy_aero_device_tables(AeroDeviceTables* t) {
   if (!t) return;
+  for (AeroLanes& l : t->lanes) destroy_lane_tables(l.lanes);
   if (t->allocation) {
     int prev = 0;
     cudaGetDevice(&prev);
@@ -79,6 +81,21 @@ AeroDeviceTables* aero_tables_for(const tchem_gb_aero* aero, int dev) {
   if (static_cast<int>(a->device_tables.size()) <= dev) a->device_tables.resize(dev + 1, nullptr);
   if (!a->device_tables[dev]) a->device_tables[dev] = upload_aero_tables(*a, dev);
   return a->device_tables[dev];
+}
+
+// The batched kernel's streams for this mechanism and particle count (built on first use).
+const LaneTables* aero_lanes_for(const tchem_gb_aero* aero, const HostTables& ht, const AeroDev& A, int dev) {
+  auto* a = const_cast<tchem_gb_aero*>(aero);
+  std::lock_guard<std::mutex> lk(a->mu);
+  AeroDeviceTables& t = *a->device_tables[dev];
+  for (const AeroLanes& l : t.lanes)
+    if (l.n_particles == A.nP && l.signature == ht.signature) return l.lanes;
+  AeroLanes l;
+  l.signature = ht.signature;
+  l.n_particles = A.nP;
+  l.lanes = upload_aero_lane_tables(ht, A, a->simpol_index.data(), dev, device_info(dev).max_smem_optin);
+  t.lanes.push_back(l);
+  return l.lanes;
 }
 
 const HostTables* host_tables_of(const tchem_gb_mech* mech) {
@@ -226,11 +243,15 @@ int tchem_gb_aero_time_advance(const tchem_gb_mech* mech, const tchem_gb_aero* a
   int dev = 0;
   cudaGetDevice(&dev);
   AeroPlan plan;
+  LanePlan lanes;
   const DeviceTables* t = nullptr;
   try {
     t = tables_for(mech, dev);
     fill_pointers(A, aero_tables_for(aero, dev));
     plan = make_aero_plan(t->dev.L, A, nbatch, dev, false);
+    const DeviceInfo info = device_info(dev);
+    lanes = plan_lanes(aero_lanes_for(aero, *mech->host_tables, A, dev), LANE_AERO, lane_aero_doubles(A), info.sm_count,
+                       info.max_smem_optin, nbatch);
   } catch (const std::bad_alloc&) {
     return fail(TCHEM_GB_ERR_NOMEM, std::string(who) + ": allocation failed");
   } catch (const std::exception& e) {
@@ -272,6 +293,39 @@ int tchem_gb_aero_time_advance(const tchem_gb_mech* mech, const tchem_gb_aero* a
   P.matrix_in_smem = plan.matrix_in_smem ? 1 : 0;
   P.queue = reinterpret_cast<int32_t*>(ws);
   P.error_word = reinterpret_cast<int32_t*>(ws + 64);
+  if (lanes.shape >= 0) {
+    int32_t* redo = reinterpret_cast<int32_t*>(ws + 192);  // count, and the general kernel's own queue at 256
+    e = cudaMemsetAsync(redo, 0, 128, stream);
+    if (e != cudaSuccess) return cuda_fail(e, "cudaMemsetAsync(workspace)");
+    LaneParams LP{};
+    LP.a.mech = P.mech;
+    LP.a.rate_param[0] = P.mech.rate_param;
+    for (int i = 0; i < kMaxMechs; ++i) LP.a.slot_of_mech[i] = i == 0 ? 0 : -1;
+    LP.a.n_items = nbatch;
+    LP.a.queue = P.queue;
+    LP.a.tol_newton = tol_newton;
+    LP.a.tol_time = tol_time;
+    LP.a.tadv = tadv;
+    LP.a.state = state;
+    LP.a.state_out = state_out;
+    LP.a.t_out = t_out;
+    LP.a.dt_out = dt_out;
+    LP.a.status = status;
+    LP.a.stats = stats;
+    LP.a.state_dim = P.state_dim;
+    LP.a.error_word = P.error_word;
+    LP.p = lanes.dev;
+    LP.s = lanes.smem;
+    LP.aero = A;
+    LP.number_conc = number_conc;
+    LP.n_gas = P.n_gas;
+    LP.redo_count = redo;
+    e = launch_lanes(LP, lanes.shape, LANE_AERO, lanes.grid, stream);
+    if (e != cudaSuccess) return cuda_fail(e, "aerosol time-advance kernel launch");
+    note_launch();
+    P.redo_count = redo;
+    P.queue = reinterpret_cast<int32_t*>(ws + 256);
+  }
   e = launch_aero(P, false, plan.grid, plan.warps, plan.smem, stream);
   if (e != cudaSuccess) return cuda_fail(e, "aerosol time-advance kernel launch");
   note_launch();

@@ -164,10 +164,7 @@ struct GroupPlan {
   bool tc = false;  // the tensor-core form (kernels_tc_advance.cu)
   MixedLayout ml{};
   // the batched sparse-LU kernel runs first and leaves single samples to the kernel above
-  int lane_shape = -1;  // -1: not used
-  int lane_grid = 0;
-  LaneSmem lane_smem{};
-  LaneDev lane_dev{};
+  LanePlan lanes;
 };
 
 struct Plan {
@@ -177,37 +174,6 @@ struct Plan {
   size_t bytes = 0;
   int m_max = 0;
 };
-
-// The batched sparse-LU kernel's shape for a batch: the fewest samples per CTA (the most slots per
-// sample, the shortest round) that still hold the batch at once, else the most that one CTA per SM holds
-// (samples then follow each other through the lanes). The shape with two CTAs per SM takes longer per
-// round (51 species: 160 k cycles for 32 samples against 103 k for 16) and less per sample, so it pays
-// when its lanes are filled several times over: from twice its room (5,003 samples over 60 s: 556 ms
-// with one CTA per SM, 618 ms with two).
-void plan_lanes(GroupPlan& g, const DeviceTables& dt, const DeviceInfo& info, int nbatch) {
-  if (!dt.lanes) return;
-  const int fp64 = g.form == TCHEM_GB_FORM_PLAIN_FP64 ? 1 : 0;
-  long best = 0;
-  for (int k = kLaneShapeCount - 1; k >= 0; --k) {
-    if (!dt.lanes->valid[fp64][k]) continue;
-    const LaneShape sh = kLaneShapes[k];
-    const long room = static_cast<long>(info.sm_count) * sh.ctas * sh.S;
-    if (room <= best || (sh.ctas > 1 && nbatch < 2 * room && g.lane_shape >= 0)) continue;
-    best = room;
-    g.lane_shape = k;
-    if (room >= nbatch) break;
-  }
-  if (g.lane_shape < 0) return;
-  const LaneShape sh = kLaneShapes[g.lane_shape];
-  const LaneDev& d = dt.lanes->dev[fp64][g.lane_shape];
-  g.lane_dev = d;
-  g.lane_smem = lane_smem(g.dev.L, d.n_entries, d.n_t, d.table_bytes, sh.S, sh.P(), fp64 != 0);
-  lane_place_streams(g.lane_smem, d, lane_room(sh.ctas, info.max_smem_optin));
-  // the limit, not this plan's bytes: another group or thread may launch the same kernel with more
-  cudaFuncSetAttribute(lane_kernel(g.lane_shape, fp64 != 0), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       info.max_smem_optin);
-  g.lane_grid = std::min(info.sm_count * sh.ctas, (std::max(nbatch, 1) + sh.S - 1) / sh.S);
-}
 
 // Groups structurally identical mechanisms and sizes each group's launch.
 // e3sm: the E3SM time advance (per-sample rate constants and source terms): every rate form of
@@ -281,7 +247,8 @@ Plan make_plan(const tchem_gb_mech* const* mechs, int n_mechs, int nbatch, bool 
       g.gmat_offset = off;
       off += up256(sizeof(float) * g.gmat_elems_per_warp * static_cast<size_t>(g.grid));
       if (o.form == TCHEM_GB_FORM_MIXED || o.form == TCHEM_GB_FORM_MIXED_SIMPLIFIED)
-        plan_lanes(g, *dts[g.mechs[0]], info, nbatch);
+        g.lanes = plan_lanes(dts[g.mechs[0]]->lanes, o.form == TCHEM_GB_FORM_PLAIN_FP64 ? LANE_F64 : LANE_F32, 0,
+                             info.sm_count, info.max_smem_optin, nbatch);
       continue;
     }
     if (mixed) {
@@ -300,7 +267,8 @@ Plan make_plan(const tchem_gb_mech* const* mechs, int n_mechs, int nbatch, bool 
       g.ml = mc.ml;
       g.matrix_in_smem = true;
       g.lda = L.m;
-      if (o.form == TCHEM_GB_FORM_MIXED && tps == 0) plan_lanes(g, *dts[g.mechs[0]], info, nbatch);
+      if (o.form == TCHEM_GB_FORM_MIXED && tps == 0) g.lanes = plan_lanes(dts[g.mechs[0]]->lanes, o.form == TCHEM_GB_FORM_PLAIN_FP64 ? LANE_F64 : LANE_F32, 0,
+                             info.sm_count, info.max_smem_optin, nbatch);
       continue;
     }
     g.lda = L.m | 1;
@@ -327,7 +295,8 @@ Plan make_plan(const tchem_gb_mech* const* mechs, int n_mechs, int nbatch, bool 
       g.gmat_offset = off;
       off += up256(sizeof(double) * g.gmat_elems_per_warp * static_cast<size_t>(g.grid) * W);
     }
-    plan_lanes(g, *dts[g.mechs[0]], info, nbatch);
+    g.lanes = plan_lanes(dts[g.mechs[0]]->lanes, o.form == TCHEM_GB_FORM_PLAIN_FP64 ? LANE_F64 : LANE_F32, 0,
+                             info.sm_count, info.max_smem_optin, nbatch);
   }
   plan.bytes = off;
   return plan;
@@ -530,13 +499,13 @@ int time_advance_impl(const tchem_gb_mech* const* mechs, int n_mechs, const int3
     P.keff_in = rates.keff;
     P.src_in = rates.src;
     P.src_stride = rates.src_stride;
-    if (gp.lane_shape >= 0) {
+    if (gp.lanes.shape >= 0) {
       LaneParams LP{};
       LP.a = P;
-      LP.p = gp.lane_dev;
-      LP.s = gp.lane_smem;
+      LP.p = gp.lanes.dev;
+      LP.s = gp.lanes.smem;
       LP.redo_count = counts + 16 + g;
-      e = launch_lanes(LP, gp.lane_shape, gp.form == TCHEM_GB_FORM_PLAIN_FP64, gp.lane_grid, gs);
+      e = launch_lanes(LP, gp.lanes.shape, gp.lanes.form, gp.lanes.grid, gs);
       if (e != cudaSuccess) return cuda_fail(e, "time-advance kernel launch");
       note_launch();
       // the samples it left, if any: the general kernel, on a queue of its own

@@ -116,6 +116,8 @@ struct AeroParams {
   int32_t* status;                // [B]
   tchem_gb_sample_stats* stats;   // [B] or null
   double* omega;                  // right-hand-side mode: [B][M]
+  // Not null: only the samples with status kStatusRedo, none of them when the count is 0.
+  const int32_t* redo_count;
   double* gmat;                   // per-warp matrix slots in global memory (when not in smem)
   int64_t gmat_stride;
   int32_t lda;

@@ -12,7 +12,8 @@
 // The Jacobian is a forward difference of the RHS, column j with the step 1e-8 max(|y_j|, 1e-20),
 // as the reference's computeJacobian (computeNumericalJacobian,
 // TChem_Impl_AerosolChemistry_Problem.hpp:204-236).
-// The right-hand side itself is in aero_rhs.cuh.
+// The right-hand side itself is in aero_rhs.cuh. The time advance runs here only for what the batched
+// kernel (kernels_lanes_impl.cuh, analytic Jacobian and sparse LU) leaves.
 #include "advance.hpp"
 #include "engine.cuh"
 #include "fp64_core.cuh"
@@ -128,6 +129,7 @@ using namespace fp64;
 
 template <int NPL, bool RHS_ONLY>
 __global__ void __launch_bounds__(256, 1) aero_kernel(const __grid_constant__ AeroParams P) {
+  if (P.redo_count && *P.redo_count == 0) return;
   extern __shared__ __align__(128) unsigned char smem[];
   uint64_t* mbar = reinterpret_cast<uint64_t*>(smem);
   unsigned char* tables = smem + 16;
@@ -188,6 +190,7 @@ __global__ void __launch_bounds__(256, 1) aero_kernel(const __grid_constant__ Ae
     if (s >= P.B) break;
     tchem_gb_tadv ta{};
     if constexpr (!RHS_ONLY) {
+      if (P.redo_count && P.status[s] != kStatusRedo) continue;  // advanced by the batched kernel
       ta = P.tadv[s];
       if (P.t_out[s] >= ta.tend) {
         if (lane == 0) {

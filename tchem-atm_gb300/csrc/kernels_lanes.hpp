@@ -6,6 +6,7 @@
 #include <algorithm>
 
 #include "advance.hpp"
+#include "kernels.hpp"
 
 namespace tchem_gb {
 
@@ -13,7 +14,9 @@ namespace tchem_gb {
 // The streams in the order of their shared-memory places: what is read most often per round first.
 enum LaneStreamId { LS_NET, LS_FORWARD, LS_BACKWARD, LS_REACTIONS, LS_FACTOR, LS_MATRIX, LS_COUNT };
 struct LaneDev {
+  int32_t m, R, Q, D;         // LaneInput
   int32_t nps, nrs, n_entries, n_t, tail, zero, vec, ms;  // ms: positions before the tail
+  const int32_t* pos;         // [m] position of each species
   const int32_t* species;           // [nps][P] position | species << 16 (no species: m)
   const uint4* packets[LS_COUNT];
   int32_t packet_count[LS_COUNT];
@@ -27,7 +30,7 @@ struct LaneDev {
 
 // Byte offsets of the CTA's shared-memory sections; every array is [...][S].
 struct LaneSmem {
-  uint32_t lu, x, v, q, ctl, tol, prog, bytes;
+  uint32_t lu, x, v, q, ctl, tol, ext, prog, bytes;
   uint32_t stream[LS_COUNT];  // resident streams, 0: read from global memory
   uint32_t stage, stage_bytes;  // what is left, for chunks of the others
 };
@@ -36,6 +39,10 @@ struct LaneParams {
   AdvanceParams a;
   LaneDev p;
   LaneSmem s;
+  // gas-aerosol problem: rows [active gas, particles], the state row's constant gas species between them
+  AeroDev aero;
+  const double* number_conc;  // [B][nP]
+  int32_t n_gas;              // gas species, active and constant
   int32_t* redo_count;  // samples left to the general kernel (status kStatusRedo)
 };
 
@@ -53,7 +60,9 @@ constexpr uint32_t lane_control_bytes(int S) {
   return (static_cast<uint32_t>(S) * (8 * kLaneControlDoubles + 4 * kLaneControlInts) + 16 + 15) & ~15u;
 }
 
-inline LaneSmem lane_smem(const MechLayout& L, int n_entries, int n_t, int table_bytes, int S, int P, bool fp64) {
+// m rows, Q rows of q, D slots of d; ext: doubles per sample of the aerosol problem (else 0).
+inline LaneSmem lane_smem(int m, int Q, int D, int ext, int n_entries, int n_t, int table_bytes, int S, int P,
+                          bool fp64) {
   auto up16 = [](size_t b) { return static_cast<uint32_t>((b + 15) & ~size_t(15)); };
   const size_t t = fp64 ? 8 : 4;
   LaneSmem s{};
@@ -61,18 +70,20 @@ inline LaneSmem lane_smem(const MechLayout& L, int n_entries, int n_t, int table
   s.lu = o;
   o += up16(t * S * n_entries);
   s.x = o;
-  o += up16(sizeof(double) * S * (L.m + 1));
+  o += up16(sizeof(double) * S * (m + 1));
   s.v = o;
-  if (!fp64) o += up16(sizeof(double) * S * (L.m + 1));
+  if (!fp64) o += up16(sizeof(double) * S * (m + 1));
   // q and, in its place at other times, the factor-slot derivatives, the tail's pivot rows and
   // columns (two of each, double-buffered), and the warps' sums of the two norms
   s.q = o;
-  o += up16(S * std::max(std::max(sizeof(double) * (L.R + 1), t * (L.NF + 1)),
+  o += up16(S * std::max(std::max(sizeof(double) * (Q + 1), t * (D + 1)),
                          std::max(t * 8 * n_t, sizeof(double) * (2 * (P * S / 32) + 1))));
   s.ctl = o;
   o += lane_control_bytes(S);
   s.tol = o;  // step tolerances by position, the same for every sample
-  o += up16(2 * sizeof(double) * L.m);
+  o += up16(2 * sizeof(double) * m);
+  s.ext = o;
+  o += up16(sizeof(double) * S * ext);
   s.prog = o;  // LaneDev::table
   o += static_cast<uint32_t>(table_bytes);
   s.bytes = o;
@@ -100,7 +111,12 @@ inline void lane_place_streams(LaneSmem& s, const LaneDev& d, uint32_t room) {
   s.bytes += s.stage_bytes;
 }
 
-const void* lane_kernel(int shape, bool fp64);
-cudaError_t launch_lanes(const LaneParams& P, int shape, bool fp64, int grid, cudaStream_t stream);
+enum LaneForm { LANE_F32 = 0, LANE_F64 = 1, LANE_AERO = 2 };  // the aerosol problem is FP64
+constexpr int kLaneForms = 3;
+inline bool lane_has_shape(LaneForm form, int shape) { return form != LANE_AERO || kLaneShapes[shape].S <= 8; }
+const void* lane_kernel(int shape, LaneForm form);
+cudaError_t launch_lanes(const LaneParams& P, int shape, LaneForm form, int grid, cudaStream_t stream);
+// Doubles per sample of the aerosol problem's own section.
+inline int lane_aero_doubles(const AeroDev& A) { return 4 * A.nS + 6 * A.nP + 4 * A.nP * A.nS; }
 
 }  // namespace tchem_gb

@@ -1,0 +1,4 @@
+// One shape of the batched sparse-LU time advance: the gas-aerosol problem, 4 samples per CTA.
+#include "kernels_lanes_impl.cuh"
+
+TCHEM_GB_LANE_SHAPE(aero_4, double, 4, 16, 1, true)

@@ -34,6 +34,7 @@
 
 #include <cstdint>
 
+#include "aero_rhs.cuh"
 #include "engine.cuh"
 #include "kernels_lanes.hpp"
 #include "lane_program.hpp"
@@ -132,7 +133,8 @@ __device__ __forceinline__ uint32_t load_byte(uint32_t at) {
   return v;
 }
 
-template <typename T, int S, int W>
+// AERO: the gas-aerosol problem (T = double): rows of q and slots of d beyond the reactions'.
+template <typename T, int S, int W, bool AERO>
 struct Kernel {
   static constexpr int NT = 32 * W;
   static constexpr int SPW = 32 / S;  // slots per warp
@@ -166,7 +168,6 @@ struct Kernel {
   __device__ __forceinline__ int& flag(int k) const {
     return reinterpret_cast<int*>(sm + K.s.ctl + S * (D_COUNT * sizeof(double) + I_COUNT * sizeof(int)))[k];
   }
-  __device__ __forceinline__ int m() const { return K.a.mech.L.m; }
 
   // This slot's packets of a stream, a warp's rounds SPW apart: in shared memory where it is resident.
   __device__ __forceinline__ const uint4* packets(int id, int& rounds) const {
@@ -515,7 +516,7 @@ struct Kernel {
     for (int k = 0; k < NRS; ++k) {
       if (k >= K.p.nrs) break;
       const uint4 f = p[k * SPW];
-      if (k * P + slot < K.a.mech.L.R) {
+      if (k * P + slot < K.p.R) {
         double v = keff[k] * x.load((f.x & 0xffffu) * S);
         if ((f.y >> 16) > 1) v *= x.load((f.x >> 16) * S);
         if ((f.y >> 16) > 2) v *= x.load((f.y & 0xffffu) * S);
@@ -533,7 +534,7 @@ struct Kernel {
     for (int k = 0; k < NRS; ++k) {
       if (k >= K.p.nrs) break;
       const uint4 f = p[k * SPW];
-      if (k * P + slot < K.a.mech.L.R) {
+      if (k * P + slot < K.p.R) {
         const int a = (f.x & 0xffffu) * S, b = (f.x >> 16) * S, c = (f.y & 0xffffu) * S, n = f.y >> 16;
         double d = n > 0 ? v.load(a) : 0.0;
         if (n >= 2) {
@@ -577,7 +578,7 @@ struct Kernel {
     for (int k = 0; k < NRS; ++k) {
       if (k >= K.p.nrs) break;
       const uint4 f = p[k * SPW];
-      if (k * P + slot < K.a.mech.L.R) {
+      if (k * P + slot < K.p.R) {
         const int n = f.y >> 16;
         const uint32_t o = f.z * S;
         if (n == 1) {
@@ -595,6 +596,99 @@ struct Kernel {
           }
         }
       }
+    }
+  }
+
+  // ---- gas-aerosol problem ----
+  // The section holds, per sample: simc [nS][4] (accommodation coefficient, mean free path, partitioning
+  // constant, kg m-3 -> ppm), nc [nP], part [nP][5] (radius, mean molecular weight, mass, moles, r / 3V),
+  // tr [nP nS][4] (condensation coefficient, and the factors of 1 / density, 1 / molecular weight and the
+  // entry's own species in the transfer's derivative by a species of the particle).
+  __device__ __forceinline__ double* ext(int i) const { return reinterpret_cast<double*>(sm + K.s.ext) + i * S + s; }
+  __device__ __forceinline__ int nc_at() const { return 4 * K.aero.nS; }
+  __device__ __forceinline__ int part_at() const { return 4 * K.aero.nS + K.aero.nP; }
+  __device__ __forceinline__ int tr_at() const { return 4 * K.aero.nS + 6 * K.aero.nP; }
+
+  // Temperature and pressure terms and number concentrations of the new sample in lane c, by all threads.
+  __device__ __forceinline__ void aero_setup_sample(int c, int smp, double p, double Tk) const {
+    const AeroDev& A = K.aero;
+    double* e = reinterpret_cast<double*>(sm + K.s.ext) + c;
+    for (int is = threadIdx.x; is < A.nS; is += NT) {
+      double sc[4];
+      fp64::aero_entry_terms(A.sim_idx + 3 * is, A.sim_par + 7 * is, Tk, p, sc);
+      for (int i = 0; i < 4; ++i) e[(4 * is + i) * S] = sc[i];
+    }
+    for (int ip = threadIdx.x; ip < A.nP; ip += NT)
+      e[(nc_at() + ip) * S] = K.number_conc[static_cast<size_t>(smp) * A.nP + ip];
+  }
+  __device__ __forceinline__ double ode(int i) const { return xs()[__ldg(K.p.pos + i) * S]; }
+
+  // Radius, mean molecular weight and mass of the particles: src/core/impl/TChem_Impl_SingleParticleUtils.hpp:50-170.
+  __device__ __forceinline__ void aero_particles() const {
+    const AeroDev& A = K.aero;
+    for (int ip = slot; ip < A.nP; ip += P) {
+      const int first = A.m_gas + ip * A.nA;
+      double volume = A.vol0, mass = A.mass0, moles = A.moles0;
+      for (int k = 0; k < A.nA; ++k) {
+        const double x = ode(first + k);
+        volume += x / A.density[k];
+        mass += x;
+        moles += x / A.mw[k];
+      }
+      const double radius = pow(volume * 3.0 / 4.0 / fp64::kAeroPi, 1.0 / 3.0);
+      const int o = part_at() + 5 * ip;
+      *ext(o) = radius;
+      *ext(o + 1) = mass / moles;
+      *ext(o + 2) = mass;
+      *ext(o + 3) = moles;
+      *ext(o + 4) = radius / (3.0 * volume);
+    }
+  }
+
+  // The (particle, entry) pairs' rows of q: src/core/impl/TChem_Impl_SIMPOL_phase_transfer.hpp:60-150, and the
+  // terms of their derivatives.
+  __device__ __forceinline__ void aero_transfers() const {
+    const AeroDev& A = K.aero;
+    double* q = qs();
+    for (int e = slot; e < A.nP * A.nS; e += P) {
+      const int ip = e / A.nS, is = e - ip * A.nS, o = part_at() + 5 * ip;
+      const double alpha = *ext(4 * is), mfp = *ext(4 * is + 1), keq = *ext(4 * is + 2), D = A.sim_par[7 * is + 4];
+      const double radius = *ext(o), avg_mw = *ext(o + 1), mass = *ext(o + 2), moles = *ext(o + 3);
+      const double kn = mfp / radius;
+      const double num = 0.75 * alpha * (1.0 + kn), den = kn * kn + (1.0 + 0.283 * alpha) * kn + 0.75 * alpha;
+      const double ffs = num / den;
+      double cond = 4.0 * fp64::kAeroPi * radius * D * ffs;
+      double evap = cond * 1.0 * (keq * avg_mw / mass);
+      const double xg = ode(A.sim_idx[3 * is + 1]), xa = ode(A.sim_idx[3 * is] + ip * A.nA);
+      // d cond / dr: radius enters directly and through kn = mfp / radius
+      const double dffs = (0.75 * alpha * den - num * (2.0 * kn + 1.0 + 0.283 * alpha)) / (den * den);
+      const double dcond = 4.0 * fp64::kAeroPi * D * (ffs - kn * dffs), keq_m = keq / moles;
+      const int t = tr_at() + 4 * e;
+      *ext(t) = cond;
+      *ext(t + 1) = dcond * *ext(o + 4) * (xg - keq_m * xa);
+      *ext(t + 2) = cond * keq_m * xa / moles;
+      *ext(t + 3) = -cond * keq_m;
+      cond *= xg;
+      evap *= xa;
+      const double d = -evap + cond;
+      q[(K.p.R + 2 * e) * S] = -*ext(nc_at() + ip) * d;
+      q[(K.p.R + 2 * e + 1) * S] = d / *ext(4 * is + 3);
+    }
+  }
+
+  // The pairs' slots of d.
+  __device__ __forceinline__ void aero_slots() const {
+    const AeroDev& A = K.aero;
+    T* d = ds() + (K.p.D - 2 * A.nP * A.nS * (1 + A.nA)) * S;
+    for (int i = slot; i < A.nP * A.nS * (1 + A.nA); i += P) {
+      const int e = i / (1 + A.nA), c = i - e * (1 + A.nA), ip = e / A.nS, is = e - ip * A.nS, t = tr_at() + 4 * e;
+      double v = *ext(t);
+      if (c > 0) {
+        v = *ext(t + 1) / A.density[c - 1] + *ext(t + 2) / A.mw[c - 1];
+        if (A.sim_idx[3 * is] - A.m_gas == c - 1) v += *ext(t + 3);
+      }
+      d[2 * i * S] = -*ext(nc_at() + ip) * v;
+      d[(2 * i + 1) * S] = v / *ext(4 * is + 3);
     }
   }
 
@@ -701,8 +795,8 @@ struct Kernel {
 
   __device__ void run() {
     const AdvanceParams& A = K.a;
-    const MechLayout& L = A.mech.L;
-    const int mm = m();
+    const int mm = K.p.m;
+    const int mg = AERO ? K.aero.m_gas : mm, nc = AERO ? K.n_gas - mg : A.state_dim - 3 - mm;  // gas, constant gas
     const double gamma = 2.0 - sqrt(2.0);
     const double cg = 1.0 / (gamma * (2.0 - gamma));
     const double cn = (1.0 - gamma) * (1.0 - gamma) / (gamma * (2.0 - gamma));
@@ -718,6 +812,7 @@ struct Kernel {
     for (int k = 0; k < NPS; ++k) sps[k] = k < K.p.nps ? __ldg(K.p.species + k * P + slot) : mm;
     auto pos = [&](int k) { return sps[k] & 0xffff; };
     auto species = [&](int k) { return sps[k] >> 16; };
+    auto column = [&](int k) { return 3 + (sps[k] >> 16) + (AERO && (sps[k] >> 16) >= mg ? nc : 0); };  // of the state row
     auto has = [&](int k) { return (sps[k] & 0xffff) < mm; };
     // the iterate itself is x
     double yn[NPS], fn[NPS], fg[NPS], rv[NPS], keff[NRS];
@@ -821,17 +916,18 @@ struct Kernel {
           const double p = row[1], Tk = row[2], t_1 = 1.0 / Tk, conv = A.mech.conv_ppm * p * t_1;
           const double* rp = A.keff_in ? nullptr : A.rate_param[ci(I_SLOT, c)];
           double* q = reinterpret_cast<double*>(sm + K.s.q) + c;
-          for (int r = threadIdx.x; r < L.R; r += NT) {
+          for (int r = threadIdx.x; r < K.p.R; r += NT) {
             double k;
             if (A.keff_in) {
-              k = A.keff_in[static_cast<size_t>(smp) * L.R + r];
+              k = A.keff_in[static_cast<size_t>(smp) * K.p.R + r];
             } else {
               k = rate_constant(A.mech.rate_type[r], rp + 8 * r, A.mech.conv_exp[r], Tk, t_1, p, conv);
-              for (int e = A.mech.cf_ptr[r]; e < A.mech.cf_ptr[r + 1]; ++e) k *= row[3 + mm + A.mech.cf_idx[e]];
+              for (int e = A.mech.cf_ptr[r]; e < A.mech.cf_ptr[r + 1]; ++e) k *= row[3 + mg + A.mech.cf_idx[e]];
             }
             if (A.k_scale) k *= A.k_scale[r];
             q[r * S] = k;
           }
+          if constexpr (AERO) aero_setup_sample(c, smp, p, Tk);
         }
         __syncthreads();
         if (!any) {
@@ -846,13 +942,13 @@ struct Kernel {
           const uint4* rx = packets(LS_REACTIONS, n_rounds);
 #pragma unroll
           for (int k = 0; k < NRS; ++k)
-            if (k < K.p.nrs && k * P + slot < L.R) {
+            if (k < K.p.nrs && k * P + slot < K.p.R) {
               keff[k] = qs()[rx[k * SPW].w * S];
               kt[k] = static_cast<T>(keff[k]);
             }
 #pragma unroll
           for (int k = 0; k < NPS; ++k) {
-            yn[k] = has(k) ? row[3 + species(k)] : 0.0;
+            yn[k] = has(k) ? row[column(k)] : 0.0;
             if (has(k)) xs()[pos(k) * S] = yn[k];
             fn[k] = fg[k] = rv[k] = 0.0;
           }
@@ -872,12 +968,17 @@ struct Kernel {
         for (int k = 0; k < NPS; ++k)
           if (has(k)) xs()[pos(k) * S] = yn[k];
       }
-      if (slot == 0) qs()[L.R * S] = 0.0;
+      if (slot == 0) qs()[K.p.Q * S] = 0.0;
       double src[NPS];
 #pragma unroll
       for (int k = 0; k < NPS; ++k) src[k] = has(k) ? __ldg(srcp + species(k)) : 0.0;
       __syncthreads();
       rates(keff);
+      if constexpr (AERO) {
+        aero_particles();
+        __syncthreads();
+        aero_transfers();
+      }
       const int step_pending = __syncthreads_or(code == C_STEP || code == C_DONE);
       double f[NPS];
       net(f);
@@ -976,10 +1077,10 @@ struct Kernel {
             const bool at_y = ci(I_ACC, s) != 0;  // else y_n: the last attempt was rejected, or no step was taken
             const double* row = A.state + static_cast<size_t>(smp) * A.state_dim;
             double* out = A.state_out + static_cast<size_t>(smp) * A.state_dim;
-            for (int i = slot; i < A.state_dim - 3 - mm; i += P) out[3 + mm + i] = row[3 + mm + i];
+            for (int i = slot; i < nc; i += P) out[3 + mg + i] = row[3 + mg + i];
 #pragma unroll
             for (int k = 0; k < NPS; ++k)
-              if (has(k)) out[3 + species(k)] = status != TCHEM_GB_SAMPLE_OK ? 0.0 : (at_y ? xs()[pos(k) * S] : yn[k]);
+              if (has(k)) out[column(k)] = status != TCHEM_GB_SAMPLE_OK ? 0.0 : (at_y ? xs()[pos(k) * S] : yn[k]);
             if (slot == 0) {
               const double rho = row[0], p = row[1], Tk = row[2];
               out[0] = rho;
@@ -1071,7 +1172,8 @@ struct Kernel {
       }
       __syncthreads();
       factor_slots(kt);
-      if (slot == 0) ds()[L.NF * S] = T(0);
+      if constexpr (AERO) aero_slots();
+      if (slot == 0) ds()[K.p.D * S] = T(0);
       __syncthreads();
       matrix(static_cast<T>(coef));
       if constexpr (kRefine) {
@@ -1095,7 +1197,7 @@ struct Kernel {
             g[k] = vs()[pos(k) * S];
             vs()[pos(k) * S] = dx[k];
           }
-        if (slot == 0) qs()[L.R * S] = 0.0;
+        if (slot == 0) qs()[K.p.Q * S] = 0.0;
         __syncthreads();
         rate_derivatives(keff);
         __syncthreads();
@@ -1179,25 +1281,25 @@ struct Kernel {
 namespace tchem_gb {
 namespace lanes {
 
-template <typename T, int S, int W, int CTAS>
+template <typename T, int S, int W, int CTAS, bool AERO>
 __global__ void __launch_bounds__(32 * W, CTAS) trbdf2_lanes_kernel(const __grid_constant__ LaneParams K) {
   extern __shared__ __align__(128) unsigned char smem[];
   constexpr int SPW = 32 / S;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  Kernel<T, S, W> k{K, smem, lane % S, lane / S, warp * SPW + lane / S, warp, 0};
+  Kernel<T, S, W, AERO> k{K, smem, lane % S, lane / S, warp * SPW + lane / S, warp, 0};
   k.run();
 }
 
 }  // namespace lanes
 }  // namespace tchem_gb
 
-#define TCHEM_GB_LANE_SHAPE(NAME, T, S, W, C)                                                         \
+#define TCHEM_GB_LANE_SHAPE(NAME, T, S, W, C, A)                                                       \
   namespace tchem_gb {                                                                              \
   const void* lane_kernel_##NAME() {                                                                \
-    return reinterpret_cast<const void*>(&lanes::trbdf2_lanes_kernel<T, S, W, C>);                       \
+    return reinterpret_cast<const void*>(&lanes::trbdf2_lanes_kernel<T, S, W, C, A>);                       \
   }                                                                                                 \
   cudaError_t launch_lanes_##NAME(const LaneParams& P, int grid, cudaStream_t stream) {              \
-    lanes::trbdf2_lanes_kernel<T, S, W, C><<<grid, 32 * W, P.s.bytes, stream>>>(P);                      \
+    lanes::trbdf2_lanes_kernel<T, S, W, C, A><<<grid, 32 * W, P.s.bytes, stream>>>(P);                      \
     return cudaGetLastError();                                                                      \
   }                                                                                                 \
   }

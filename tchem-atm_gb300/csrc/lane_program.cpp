@@ -219,16 +219,46 @@ LaneStream interleave(const std::vector<std::vector<Packet>>& slot, int warps, c
 
 }  // namespace
 
-LanePattern build_lane_pattern(const HostTables& ht) {
+LaneInput lane_input(const HostTables& ht) {
   const MechLayout& L = ht.L;
-  const int m = L.m;
+  LaneInput in;
+  in.m = L.m;
+  in.R = in.Q = L.R;
+  in.D = L.NF;
+  in.max_factors = L.max_factors;
+  const int32_t* rf_ptr = section<int32_t>(ht, L.off_rf_ptr);
+  const int16_t* rf_sp = section<int16_t>(ht, L.off_rf_sp);
+  in.rf_ptr.assign(rf_ptr, rf_ptr + L.R + 1);
+  in.rf_sp.assign(rf_sp, rf_sp + L.NF);
+  const int32_t* pr_ptr = section<int32_t>(ht, L.off_pr_ptr);
+  const int16_t* pr_r = section<int16_t>(ht, L.off_pr_r);
+  const double* pr_nu = section<double>(ht, L.off_pr_nu);
+  in.net.resize(L.m);
+  for (int i = 0; i < L.m; ++i)
+    for (int e = pr_ptr[i]; e < pr_ptr[i + 1]; ++e) in.net[i].push_back({pr_r[e], pr_nu[e]});
+  const int32_t* rc = section<int32_t>(ht, L.off_jz_rc);
+  const int32_t* jz_ptr = section<int32_t>(ht, L.off_jz_ptr);
+  const int16_t* jc_f = section<int16_t>(ht, L.off_jc_f);
+  const double* jc_nu = section<double>(ht, L.off_jc_nu);
+  for (int z = 0; z < L.NZ; ++z) {
+    LaneInput::Entry e{rc[z] >> 16, rc[z] & 0xffff, {}};
+    for (int c = jz_ptr[z]; c < jz_ptr[z + 1]; ++c) e.terms.push_back({jc_f[c], jc_nu[c]});
+    in.jac.push_back(std::move(e));
+  }
+  const double* emis = section<double>(ht, L.off_emis);
+  in.emis.assign(emis, emis + L.m);
+  return in;
+}
+
+LanePattern build_lane_pattern(const LaneInput& in) {
+  const int m = in.m;
   if (m > kLaneMaxSpecies) throw std::domain_error("lane program: too many species");
-  if (L.max_factors > 3) throw std::domain_error("lane program: more than three reactant factors");
+  if (in.Q > 0xffff || in.D >= 0xffff) throw std::domain_error("lane program: too many rates");
+  if (in.max_factors > 3) throw std::domain_error("lane program: more than three reactant factors");
   std::vector<char> A(static_cast<size_t>(m) * m, 0);
   auto at = [&](int i, int j) -> char& { return A[static_cast<size_t>(i) * m + j]; };
   for (int i = 0; i < m; ++i) at(i, i) = 1;
-  const int32_t* rc = section<int32_t>(ht, L.off_jz_rc);
-  for (int z = 0; z < L.NZ; ++z) at(rc[z] >> 16, rc[z] & 0xffff) = 1;
+  for (const auto& e : in.jac) at(e.row, e.col) = 1;
   LanePattern p;
   p.m = m;
   // Greedy Markowitz on the diagonal, several independent pivots at a time: every remaining species
@@ -290,7 +320,7 @@ int lane_entries(const LanePattern& pat, int P, int n_t) {
 // instructions over four schedulers; latency: a level's barrier and dependent loads about 250 cycles, a
 // tail step about 250. FP64 has no tail: the inverse needs three times the products of the triangular
 // factors, on a pipe of 2 per cycle.
-int lane_tail_size(const MechLayout& L, const LanePattern& pat, const LaneShape& shape, bool fp64) {
+int lane_tail_size(const LaneInput& in, const LanePattern& pat, const LaneShape& shape, bool fp64) {
   if (fp64) return 0;
   const int S = shape.S, warps = shape.warps;
   const int m = pat.m, P = shape.P(), gr = lane_grid_rows(P), gc = lane_grid_cols(P);
@@ -324,7 +354,7 @@ int lane_tail_size(const MechLayout& L, const LanePattern& pat, const LaneShape&
     const double step = tr * tc + 3.0 * (tr + tc) + 40.0;
     const double issue = (35.0 * rows + n_t * warps * step) / 4.0;
     const double latency = 250.0 * n_lv * (2 + 2 * solves) + 250.0 * n_t;
-    const uint32_t bytes = lane_smem(L, lane_entries(pat, P, n_t), n_t, shape.ctas > 1 ? 704 : 2048, S, P, false).bytes;
+    const uint32_t bytes = lane_smem(in.m, in.Q, in.D, 0, lane_entries(pat, P, n_t), n_t, shape.ctas > 1 ? 704 : 2048, S, P, false).bytes;
     if (bytes > lane_room(shape.ctas, 227 * 1024) && c >= 0) continue;
     const double cost = issue + latency;
     if (c < 0 || cost < best_cost) {
@@ -335,9 +365,8 @@ int lane_tail_size(const MechLayout& L, const LanePattern& pat, const LaneShape&
   return best;
 }
 
-LaneProgram build_lane_program(const HostTables& ht, const LanePattern& pat, int P, int warps, int n_t, bool fp64) {
-  const MechLayout& L = ht.L;
-  const int m = L.m, R = L.R;
+LaneProgram build_lane_program(const LaneInput& in, const LanePattern& pat, int P, int warps, int n_t, bool fp64) {
+  const int m = in.m, R = in.R;
   const int ms = std::max(0, m - n_t);  // sparse positions; tail row i is position ms + i
   LaneProgram lp;
   lp.m = m;
@@ -368,8 +397,7 @@ LaneProgram build_lane_program(const HostTables& ht, const LanePattern& pat, int
   const int zero = lp.zero, vec = lp.vec, n_entries = lp.n_entries;
 
   // ---- reactions: most factors first, dealt to the slots in turn ----
-  const int32_t* rf_ptr = section<int32_t>(ht, L.off_rf_ptr);
-  const int16_t* rf_sp = section<int16_t>(ht, L.off_rf_sp);
+  const std::vector<int32_t>&rf_ptr = in.rf_ptr, &rf_sp = in.rf_sp;
   std::vector<int> ro(R);
   std::iota(ro.begin(), ro.end(), 0);
   std::stable_sort(ro.begin(), ro.end(),
@@ -391,13 +419,10 @@ LaneProgram build_lane_program(const HostTables& ht, const LanePattern& pat, int
   }
 
   // ---- species: longest net-production lists first, dealt to the slots in turn and back ----
-  const int32_t* pr_ptr = section<int32_t>(ht, L.off_pr_ptr);
-  const int16_t* pr_r = section<int16_t>(ht, L.off_pr_r);
-  const double* pr_nu = section<double>(ht, L.off_pr_nu);
   std::vector<int> so(m);
   std::iota(so.begin(), so.end(), 0);
   std::stable_sort(so.begin(), so.end(),
-                   [&](int a, int b) { return pr_ptr[a + 1] - pr_ptr[a] > pr_ptr[b + 1] - pr_ptr[b]; });
+                   [&](int a, int b) { return in.net[a].size() > in.net[b].size(); });
   std::vector<int> slot_species(static_cast<size_t>(lp.nps) * P, -1);
   lp.species.assign(static_cast<size_t>(lp.nps) * P, m);
   for (int q = 0; q < m; ++q) {
@@ -411,20 +436,20 @@ LaneProgram build_lane_program(const HostTables& ht, const LanePattern& pat, int
     // one segment per species of the slot, as long as the warp's longest list, a multiple of 2
     const int spw = P / warps;
     std::vector<std::vector<Packet>> slot(P);
-    const Packet none{{static_cast<uint32_t>(R), 0u, 0u, 0u}};
+    const Packet none{{static_cast<uint32_t>(in.Q), 0u, 0u, 0u}};  // q[Q] = 0
     for (int w = 0; w < warps; ++w)
       for (int k = 0; k < kLaneSegments; ++k) {
         size_t n = 0;
         for (int s = w * spw; s < (w + 1) * spw && k < lp.nps; ++s) {
           const int sp = slot_species[static_cast<size_t>(k) * P + s];
           if (sp < 0) continue;
-          for (int e = pr_ptr[sp]; e < pr_ptr[sp + 1]; ++e) {
+          for (const auto& t : in.net[sp]) {
             Packet p{};
-            p.w[0] = static_cast<uint32_t>(pr_r[e]);
-            std::memcpy(&p.w[2], &pr_nu[e], sizeof(double));
+            p.w[0] = static_cast<uint32_t>(t.first);
+            std::memcpy(&p.w[2], &t.second, sizeof(double));
             slot[s].push_back(p);
           }
-          n = std::max<size_t>(n, pr_ptr[sp + 1] - pr_ptr[sp]);
+          n = std::max(n, in.net[sp].size());
         }
         n += n % 2;
         const size_t end = (k ? lp.net_end[w * kLaneSegments + k - 1] : 0) + n;
@@ -436,14 +461,10 @@ LaneProgram build_lane_program(const HostTables& ht, const LanePattern& pat, int
 
   // ---- matrix: the nonzeros of J and the diagonal, longest contribution lists first ----
   {
-    const int32_t* rc = section<int32_t>(ht, L.off_jz_rc);
-    const int32_t* jz_ptr = section<int32_t>(ht, L.off_jz_ptr);
-    const int16_t* jc_f = section<int16_t>(ht, L.off_jc_f);
-    const double* jc_nu = section<double>(ht, L.off_jc_nu);
     std::vector<std::vector<std::pair<int, double>>> list(zero);
-    for (int z = 0; z < L.NZ; ++z) {
-      auto& l = list[E(pat.pos[rc[z] >> 16], pat.pos[rc[z] & 0xffff])];
-      for (int c = jz_ptr[z]; c < jz_ptr[z + 1]; ++c) l.push_back({jc_f[c], jc_nu[c]});
+    for (const auto& e : in.jac) {
+      auto& l = list[E(pat.pos[e.row], pat.pos[e.col])];
+      l.insert(l.end(), e.terms.begin(), e.terms.end());
     }
     std::vector<char> diag(zero, 0);
     for (int k = 0; k < ms; ++k) diag[k] = 1;
@@ -451,7 +472,7 @@ LaneProgram build_lane_program(const HostTables& ht, const LanePattern& pat, int
     std::vector<int> eo(zero);
     std::iota(eo.begin(), eo.end(), 0);
     std::stable_sort(eo.begin(), eo.end(), [&](int a, int b) { return list[a].size() > list[b].size(); });
-    const uint32_t dz = static_cast<uint32_t>(L.NF);  // d[NF] = 0
+    const uint32_t dz = static_cast<uint32_t>(in.D);  // d[D] = 0
     const int per = fp64 ? 1 : 2;
     std::vector<std::vector<Packet>> slot(P);
     std::priority_queue<std::pair<int, int>, std::vector<std::pair<int, int>>, std::greater<>> load;

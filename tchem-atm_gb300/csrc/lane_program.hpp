@@ -107,7 +107,24 @@ struct LaneProgram {
   LaneStream matrix, factor, forward, backward;
 };
 
-// Fill and static order of a mechanism's Newton matrix.
+// What a problem is made of: reactions with their reactant factors, rows of the right-hand side as sums
+// over q (the reactions' rates and rows that the kernel computes otherwise), entries of the Jacobian as
+// sums over d (one slot per reactant factor, and further ones).
+struct LaneInput {
+  int m = 0, R = 0, Q = 0, D = 0;                // rows, reactions, rows of q, slots of d
+  int max_factors = 0;
+  std::vector<int32_t> rf_ptr, rf_sp;            // factors of reaction r; slot numbers as d
+  std::vector<std::vector<std::pair<int, double>>> net;  // [m]: (row of q, coefficient)
+  struct Entry {
+    int row, col;
+    std::vector<std::pair<int, double>> terms;   // (slot of d, coefficient)
+  };
+  std::vector<Entry> jac;
+  std::vector<double> emis;                      // [m]
+};
+LaneInput lane_input(const HostTables& ht);
+
+// Fill and static order of a problem's Newton matrix.
 struct LanePattern {
   int m = 0;
   std::vector<int32_t> order, pos;
@@ -115,10 +132,10 @@ struct LanePattern {
 };
 
 // Throws std::domain_error where the encoding does not cover the mechanism.
-LanePattern build_lane_pattern(const HostTables& ht);
+LanePattern build_lane_pattern(const LaneInput& in);
 // The tail size for a shape, and the program.
-int lane_tail_size(const MechLayout& L, const LanePattern& pat, const LaneShape& shape, bool fp64);
-LaneProgram build_lane_program(const HostTables& ht, const LanePattern& pat, int P, int warps, int n_t, bool fp64);
+int lane_tail_size(const LaneInput& in, const LanePattern& pat, const LaneShape& shape, bool fp64);
+LaneProgram build_lane_program(const LaneInput& in, const LanePattern& pat, int P, int warps, int n_t, bool fp64);
 // Entries (pattern, tail block, zero, vector section) for a tail size, without building the program.
 int lane_entries(const LanePattern& pat, int P, int n_t);
 

@@ -29,38 +29,38 @@ struct Arena {
   }
 };
 
-}  // namespace
-
-LaneTables* upload_lane_tables(const HostTables& ht, int device, int max_smem) {
+// Streams of the forms [first, last] of one problem.
+LaneTables* upload(const LaneInput& in, int ext, int first, int last, int device, int max_smem) {
   LanePattern pat;
   try {
-    pat = build_lane_pattern(ht);
+    pat = build_lane_pattern(in);
   } catch (const std::domain_error&) {
     return nullptr;
   }
   struct Offsets {
     size_t species, table, packets[LS_COUNT];
-  } at[2][kLaneShapeCount] = {};
+  } at[kLaneForms][kLaneShapeCount] = {};
   LaneTables t;
   Arena arena;
-  const size_t emis = arena.put(reinterpret_cast<const double*>(ht.blob.data() + ht.L.off_emis),
-                                static_cast<size_t>(ht.L.m));
+  const size_t emis = arena.put(in.emis), pos = arena.put(pat.pos);
   bool any = false;
-  for (int fp64 = 0; fp64 < 2; ++fp64)
+  for (int form = first; form <= last; ++form)
     for (int k = 0; k < kLaneShapeCount; ++k) {
+      if (!lane_has_shape(static_cast<LaneForm>(form), k)) continue;
+      const bool fp64 = form != LANE_F32;
       const LaneShape sh = kLaneShapes[k];
-      const int n_t = lane_tail_size(ht.L, pat, sh, fp64 != 0);
-      LaneDev& d = t.dev[fp64][k];
-      if (lane_smem(ht.L, lane_entries(pat, sh.P(), n_t), n_t, 0, sh.S, sh.P(), fp64 != 0).bytes >
+      const int n_t = lane_tail_size(in, pat, sh, fp64);
+      LaneDev& d = t.dev[form][k];
+      if (lane_smem(in.m, in.Q, in.D, ext, lane_entries(pat, sh.P(), n_t), n_t, 0, sh.S, sh.P(), fp64).bytes >
           lane_room(sh.ctas, max_smem))
         continue;
       LaneProgram lp;
       try {
-        lp = build_lane_program(ht, pat, sh.P(), sh.warps, n_t, fp64 != 0);
+        lp = build_lane_program(in, pat, sh.P(), sh.warps, n_t, fp64);
       } catch (const std::domain_error&) {
         continue;
       }
-      Offsets& o = at[fp64][k];
+      Offsets& o = at[form][k];
       std::vector<int32_t> head(2 * LS_COUNT * sh.warps);
       std::vector<uint8_t> levels;
       const size_t level_base = 4 * (head.size() + lp.net_end.size());
@@ -86,12 +86,16 @@ LaneTables* upload_lane_tables(const HostTables& ht, int device, int max_smem) {
       std::memcpy(table.data() + 4 * head.size(), lp.net_end.data(), 4 * lp.net_end.size());
       if (!levels.empty()) std::memcpy(table.data() + level_base, levels.data(), levels.size());
       d.table_bytes = static_cast<int32_t>(table.size());
-      if (lane_smem(ht.L, lp.n_entries, n_t, d.table_bytes, sh.S, sh.P(), fp64 != 0).bytes >
+      if (lane_smem(in.m, in.Q, in.D, ext, lp.n_entries, n_t, d.table_bytes, sh.S, sh.P(), fp64).bytes >
           lane_room(sh.ctas, max_smem))
         continue;
       o.table = arena.put(table);
       o.species = arena.put(lp.species);
-      t.valid[fp64][k] = any = true;
+      t.valid[form][k] = any = true;
+      d.m = in.m;
+      d.R = in.R;
+      d.Q = in.Q;
+      d.D = in.D;
       d.nps = lp.nps;
       d.nrs = lp.nrs;
       d.n_entries = lp.n_entries;
@@ -115,17 +119,81 @@ LaneTables* upload_lane_tables(const HostTables& ht, int device, int max_smem) {
     throw std::runtime_error(std::string("instruction streams: ") + cudaGetErrorString(e));
   }
   const unsigned char* b = static_cast<const unsigned char*>(t.allocation);
-  for (int fp64 = 0; fp64 < 2; ++fp64)
+  for (int form = first; form <= last; ++form)
     for (int k = 0; k < kLaneShapeCount; ++k) {
-      if (!t.valid[fp64][k]) continue;
-      const Offsets& o = at[fp64][k];
-      LaneDev& d = t.dev[fp64][k];
+      if (!t.valid[form][k]) continue;
+      const Offsets& o = at[form][k];
+      LaneDev& d = t.dev[form][k];
       d.species = reinterpret_cast<const int32_t*>(b + o.species);
       d.table = reinterpret_cast<const uint4*>(b + o.table);
       for (int i = 0; i < LS_COUNT; ++i) d.packets[i] = reinterpret_cast<const uint4*>(b + o.packets[i]);
       d.emis = reinterpret_cast<const double*>(b + emis);
+      d.pos = reinterpret_cast<const int32_t*>(b + pos);
     }
   return new LaneTables(t);
+}
+
+}  // namespace
+
+LaneTables* upload_lane_tables(const HostTables& ht, int device, int max_smem) {
+  return upload(lane_input(ht), 0, LANE_F32, LANE_F64, device, max_smem);
+}
+
+LaneTables* upload_aero_lane_tables(const HostTables& ht, const AeroDev& A, const int32_t* simpol_index, int device,
+                                    int max_smem) {
+  // Each (particle, SIMPOL entry) pair is two rows of q: what its transfer takes from the gas species and
+  // gives to the aerosol species; and 2 (1 + nA) slots of d: the derivatives of the two by the gas species
+  // and by each species of the particle. The kernel computes both (aero_transfers, aero_slots).
+  LaneInput in = lane_input(ht);
+  const int R = in.R, D = in.D, nA = A.nA;
+  in.m = A.M;
+  in.net.resize(A.M);
+  in.emis.resize(A.M, 0.0);
+  for (int ip = 0; ip < A.nP; ++ip)
+    for (int is = 0; is < A.nS; ++is) {
+      const int e = ip * A.nS + is, gas = simpol_index[3 * is + 1], aero = simpol_index[3 * is] + ip * nA;
+      in.net[gas].push_back({R + 2 * e, 1.0});
+      in.net[aero].push_back({R + 2 * e + 1, 1.0});
+      for (int c = 0; c <= nA; ++c) {
+        const int col = c == 0 ? gas : A.m_gas + ip * nA + c - 1, slot = D + 2 * (e * (1 + nA) + c);
+        in.jac.push_back({gas, col, {{slot, 1.0}}});
+        in.jac.push_back({aero, col, {{slot + 1, 1.0}}});
+      }
+    }
+  in.Q = R + 2 * A.nP * A.nS;
+  in.D = D + 2 * A.nP * A.nS * (1 + nA);
+  return upload(in, lane_aero_doubles(A), LANE_AERO, LANE_AERO, device, max_smem);
+}
+
+// The batched sparse-LU kernel's shape for a batch: the fewest samples per CTA (the most slots per
+// sample, the shortest round) that still hold the batch at once, else the most that one CTA per SM holds
+// (samples then follow each other through the lanes). The shape with two CTAs per SM takes longer per
+// round (51 species: 160 k cycles for 32 samples against 103 k for 16) and less per sample, so it pays
+// when its lanes are filled several times over: from twice its room (5,003 samples over 60 s: 556 ms
+// with one CTA per SM, 618 ms with two).
+LanePlan plan_lanes(const LaneTables* t, LaneForm form, int ext, int sm_count, int max_smem, int nbatch) {
+  LanePlan p;
+  p.form = form;
+  long best = 0;
+  for (int k = kLaneShapeCount - 1; t && k >= 0; --k) {
+    if (!t->valid[form][k]) continue;
+    const LaneShape sh = kLaneShapes[k];
+    const long room = static_cast<long>(sm_count) * sh.ctas * sh.S;
+    if (room <= best || (sh.ctas > 1 && nbatch < 2 * room && p.shape >= 0)) continue;
+    best = room;
+    p.shape = k;
+    if (room >= nbatch) break;
+  }
+  if (p.shape < 0) return p;
+  const LaneShape sh = kLaneShapes[p.shape];
+  p.dev = t->dev[form][p.shape];
+  p.smem = lane_smem(p.dev.m, p.dev.Q, p.dev.D, ext, p.dev.n_entries, p.dev.n_t, p.dev.table_bytes, sh.S, sh.P(),
+                     form != LANE_F32);
+  lane_place_streams(p.smem, p.dev, lane_room(sh.ctas, max_smem));
+  // the limit, not this plan's bytes: another group or thread may launch the same kernel with more
+  cudaFuncSetAttribute(lane_kernel(p.shape, form), cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem);
+  p.grid = std::min(sm_count * sh.ctas, (std::max(nbatch, 1) + sh.S - 1) / sh.S);
+  return p;
 }
 
 void destroy_lane_tables(LaneTables* t) {
