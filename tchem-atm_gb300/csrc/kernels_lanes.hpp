@@ -60,6 +60,9 @@ constexpr uint32_t lane_control_bytes(int S) {
   return (static_cast<uint32_t>(S) * (8 * kLaneControlDoubles + 4 * kLaneControlInts) + 16 + 15) & ~15u;
 }
 
+// The tail's published rows and columns: one sample's values side by side, samples this far apart (16-byte
+// loads of eight samples then fall in distinct banks).
+constexpr int lane_publish_stride(int n_t) { return n_t + 4; }
 // m rows, Q rows of q, D slots of d; ext: doubles per sample of the aerosol problem (else 0).
 inline LaneSmem lane_smem(int m, int Q, int D, int ext, int n_entries, int n_t, int table_bytes, int S, int P,
                           bool fp64) {
@@ -77,7 +80,7 @@ inline LaneSmem lane_smem(int m, int Q, int D, int ext, int n_entries, int n_t, 
   // columns (two of each, double-buffered), and the warps' sums of the two norms
   s.q = o;
   o += up16(S * std::max(std::max(sizeof(double) * (Q + 1), t * (D + 1)),
-                         std::max(t * 8 * n_t, sizeof(double) * (2 * (P * S / 32) + 1))));
+                         std::max(t * 8 * lane_publish_stride(n_t), sizeof(double) * (2 * (P * S / 32) + 1))));
   s.ctl = o;
   o += lane_control_bytes(S);
   s.tol = o;  // step tolerances by position, the same for every sample

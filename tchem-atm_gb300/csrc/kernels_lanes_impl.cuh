@@ -349,105 +349,205 @@ struct Kernel {
   }
 
   // In-place Gauss-Jordan inverse of the tail block, no pivot search, two pivots per step: slot (pr, pc) of
-  // the grid holds rows pr + GR a and columns pc + GC c in registers. Per step the owners of the two
-  // pivot rows and columns publish them (double-buffered, one barrier); every slot solves the 2 x 2
-  // pivot block for its columns and updates its tile with both rows. A step is bound by its chain of
-  // barrier, loads and reciprocals and by the instructions around the products: two pivots share them.
+  // the grid holds rows pr TR .. and columns pc TC .. in registers. Per step the owners of the two pivot
+  // rows and columns publish them (double-buffered, one barrier); every slot solves the 2 x 2 pivot
+  // block for its columns and updates its tile with both rows. A step is bound by the instructions around
+  // the products and by its chain of barrier, loads and reciprocals: two pivots share them, a slot's
+  // stretch of a published row or column is one or two wide loads, and products go two to an instruction
+  // (fma.rn.f32x2). One pivot per step took 27.8 k cycles for 16 samples' 32 x 32 blocks, two pivots with
+  // cyclic tiles and single loads 24.0 k (one sample: 6.4 k; 160 x 160: 113 k), this 23.8 k (5.7 k; 113 k).
   template <int TR>
   __device__ __forceinline__ void invert_tail() {
     constexpr int GR = lane_grid_rows(P), GC = lane_grid_cols(P), F = GR / GC, N = TR * GR, TC = N / GC;
-    constexpr int ST = lane_tail_stride(P, N);
+    constexpr int ST = lane_tail_stride(P, N), NS = N + 4;  // lane_publish_stride
+    constexpr uint32_t kRow = NS * S * 4;                   // bytes of one published row of all samples
+    static_assert(TC % 2 == 0, "pivots go in pairs");
     const Shared<T> A{lus().at + K.p.tail * S * static_cast<uint32_t>(sizeof(T))};
-    // [2]: two rows, two columns, each [N][S]
-    const Shared<T> pub{base() + K.s.q + s * static_cast<uint32_t>(sizeof(T))};
+    const uint32_t pub = base() + K.s.q + s * NS * 4;  // [2]: two rows, two columns, each [S][NS]
     const int pr = slot / GC, pc = slot % GC;
-    T t[TR][TC];
+    uint64_t t[TR][TC / 2];  // pairs of columns
 #pragma unroll
     for (int a = 0; a < TR; ++a)
 #pragma unroll
-      for (int c = 0; c < TC; ++c) t[a][c] = A.load(((pr + GR * a) * ST + pc + GC * c) * S);
-    if (pr < 2)
-#pragma unroll
-      for (int c = 0; c < TC; ++c) pub.store((pr * N + pc + GC * c) * S, t[0][c]);
-    if (pc < 2)
-#pragma unroll
-      for (int a = 0; a < TR; ++a) pub.store(((2 + pc) * N + pr + GR * a) * S, t[a][0]);
+      for (int c = 0; c < TC / 2; ++c) {
+        const int at = (pr * TR + a) * ST + pc * TC + 2 * c;
+        t[a][c] = pack(A.load(at * S), A.load((at + 1) * S));
+      }
+    const uint32_t my_row = pub + pc * TC * 4, my_col = pub + 2 * kRow + pr * TR * 4;
+    publish_step<TR, TC>(t, my_row, my_col, pr, pc, 0, 0);
     __syncthreads();
-#pragma unroll
-    for (int blk = 0; blk < TR * F; ++blk) {
-      const int ta = blk / F, tc = blk, r0 = GC * (blk % F);  // the pivots' tile row and column, first grid row
 #pragma unroll 1
-      for (int b = 0; b < GC; b += 2) {
-        const int k = GC * blk + b;
-        constexpr uint32_t kStep = N * S * static_cast<uint32_t>(sizeof(T));
-        const Shared<T> x0{pub.at + ((k >> 1) & 1) * 4 * kStep}, x1{x0.at + kStep}, y0{x1.at + kStep}, y1{y0.at + kStep};
-        // [a b; c d] = [1 0; l 1] [a b; 0 e]
-        const T pa = x0.load(k * S), pb = x0.load((k + 1) * S), pcc = x1.load(k * S), pd = x1.load((k + 1) * S);
-        const T p0 = Num<T>::recip(pa), l = pcc * p0, w = pb * p0, e = Num<T>::mul_sub(l, pb, pd), p1 = Num<T>::recip(e);
-        T q0[TC], q1[TC], l0[TR], l1[TR], big0 = T(0), big1 = T(0);
+    for (int blk = 0; blk < GC; ++blk) {
 #pragma unroll
-        for (int c = 0; c < TC; ++c) {
-          const T u = x0.load((pc + GC * c) * S), v = x1.load((pc + GC * c) * S);
-          q1[c] = p1 * Num<T>::mul_sub(l, u, v);
-          q0[c] = Num<T>::mul_sub(w, q1[c], p0 * u);
+      for (int c0 = 0; c0 < TC; c0 += 2) {
+        // pivots k, k + 1: tile columns c0, c0 + 1 of grid column blk; tile rows and grid rows
+        constexpr int kLast = TC - 2;
+        const int k = blk * TC + c0;
+        const int buf = (k >> 1) & 1;
+        const int ra = c0 % TR, rb = (c0 + 1) % TR, ga = blk * F + c0 / TR, gb = blk * F + (c0 + 1) / TR;
+        const uint32_t x0 = my_row + buf * 4 * kRow, y0 = my_col + buf * 4 * kRow;
+        const uint32_t piv = pub + buf * 4 * kRow + k * 4;
+        // [a b; c d] = [1 0; l 1] [a b; 0 e]
+        float pa, pb, pcc, pd;
+        load_pair(piv, pa, pb);
+        load_pair(piv + kRow, pcc, pd);
+        uint64_t u[TC / 2], v[TC / 2];
+        float l0[TR], l1[TR];
+        load_row<TC>(x0, u);
+        load_row<TC>(x0 + kRow, v);
+        load_col<TR>(y0, l0);
+        load_col<TR>(y0 + kRow, l1);
+        const float p0 = Num<float>::recip(pa), l = pcc * p0, w = pb * p0, e = fmaf(-l, pb, pd), p1 = Num<float>::recip(e);
+        float big0 = 0.f, big1 = 0.f;
+#pragma unroll
+        for (int a = 0; a < TR; ++a) {
+          big0 = fmaxf(big0, fabsf(l0[a]));
+          big1 = fmaxf(big1, fabsf(fmaf(-l0[a], w, l1[a])));  // after the first elimination
+        }
+        // a multiplier beyond the bound, or a zero or non-finite pivot (its own row's multiplier is 1)
+        if (!(big0 * fabsf(p0) <= kLaneMaxGrowth) || !(big1 * fabsf(p1) <= kLaneMaxGrowth)) bad = 1;
+        if (!(fabsf(pa) > 0.f) || !(fabsf(e) > 0.f)) bad = 1;
+        // rows of the inverse of the pivot block times the pivot rows
+        const uint64_t ml = pack(-l, -l), mw = pack(-w, -w), pp0 = pack(p0, p0), pp1 = pack(p1, p1);
+#pragma unroll
+        for (int c = 0; c < TC / 2; ++c) {
+          v[c] = mul2(pp1, fma2(ml, u[c], v[c]));
+          u[c] = fma2(mw, v[c], mul2(pp0, u[c]));
+        }
+        if (pc == blk) {  // the pivot columns become the inverse's
+          const float n1 = -l * p1;
+          v[c0 / 2] = pack(n1, p1);
+          u[c0 / 2] = pack(fmaf(-w, n1, p0), -w * p1);
+#pragma unroll
+          for (int a = 0; a < TR; ++a) t[a][c0 / 2] = 0ull;
         }
 #pragma unroll
         for (int a = 0; a < TR; ++a) {
-          l0[a] = y0.load((pr + GR * a) * S);
-          l1[a] = y1.load((pr + GR * a) * S);
-          big0 = fmax(big0, fabs(l0[a]));
-          big1 = fmax(big1, fabs(Num<T>::mul_sub(l0[a], w, l1[a])));  // after the first elimination
+          const uint64_t m0 = pack(-l0[a], -l0[a]), m1 = pack(-l1[a], -l1[a]);
+#pragma unroll
+          for (int c = 0; c < TC / 2; ++c) t[a][c] = fma2(m1, v[c], fma2(m0, u[c], t[a][c]));
         }
-        // a multiplier beyond the bound, or a zero or non-finite pivot (its own row's multiplier is 1)
-        if (!(big0 * fabs(p0) <= T(kLaneMaxGrowth)) || !(big1 * fabs(p1) <= T(kLaneMaxGrowth))) bad = 1;
-        if (!(fabs(pa) > T(0)) || !(fabs(e) > T(0))) bad = 1;
-        if (pc == b || pc == b + 1) {  // the pivot columns become the inverse's
-          q1[tc] = pc == b ? -l * p1 : p1;
-          q0[tc] = Num<T>::mul_sub(w, q1[tc], pc == b ? p0 : T(0));
+        if (pr == ga) {
 #pragma unroll
-          for (int a = 0; a < TR; ++a) t[a][tc] = T(0);
+          for (int c = 0; c < TC / 2; ++c) t[ra][c] = u[c];
         }
+        if (pr == gb) {
 #pragma unroll
-        for (int a = 0; a < TR; ++a)
-#pragma unroll
-          for (int c = 0; c < TC; ++c)
-            t[a][c] = Num<T>::mul_sub(l1[a], q1[c], Num<T>::mul_sub(l0[a], q0[c], t[a][c]));
-        if (pr == r0 + b) {
-#pragma unroll
-          for (int c = 0; c < TC; ++c) t[ta][c] = q0[c];
+          for (int c = 0; c < TC / 2; ++c) t[rb][c] = v[c];
         }
-        if (pr == r0 + b + 1) {
-#pragma unroll
-          for (int c = 0; c < TC; ++c) t[ta][c] = q1[c];
-        }
-        if (b + 2 < GC) {
-          const Shared<T> n{pub.at + (((k >> 1) + 1) & 1) * 4 * kStep};
-          const int rr = pr - (r0 + b + 2), cc = pc - (b + 2);
-          if (rr == 0 || rr == 1)
-#pragma unroll
-            for (int c = 0; c < TC; ++c) n.store((rr * N + pc + GC * c) * S, t[ta][c]);
-          if (cc == 0 || cc == 1)
-#pragma unroll
-            for (int a = 0; a < TR; ++a) n.store(((2 + cc) * N + pr + GR * a) * S, t[a][tc]);
+        const uint32_t nrow = my_row + (buf ^ 1) * 4 * kRow, ncol = my_col + (buf ^ 1) * 4 * kRow;
+        if (c0 < kLast) {
+          publish_step<TR, TC>(t, nrow, ncol, pr, pc, blk, c0 + 2);
+          __syncthreads();
+        } else if (blk + 1 < GC) {
+          publish_step<TR, TC>(t, nrow, ncol, pr, pc, blk + 1, 0);
           __syncthreads();
         }
-      }
-      if (blk + 1 < TR * F) {  // the next pivots open the next tile row or column (GC / 2 is even: buffer 0)
-        const int na = (blk + 1) / F, rr = pr - GC * ((blk + 1) % F);
-        if (rr == 0 || rr == 1)
-#pragma unroll
-          for (int c = 0; c < TC; ++c) pub.store((rr * N + pc + GC * c) * S, t[na][c]);
-        if (pc < 2)
-#pragma unroll
-          for (int a = 0; a < TR; ++a) pub.store(((2 + pc) * N + pr + GR * a) * S, t[a][blk + 1]);
-        __syncthreads();
       }
     }
 #pragma unroll
     for (int a = 0; a < TR; ++a)
 #pragma unroll
-      for (int c = 0; c < TC; ++c) A.store(((pr + GR * a) * ST + pc + GC * c) * S, t[a][c]);
+      for (int c = 0; c < TC / 2; ++c) {
+        const int at = (pr * TR + a) * ST + pc * TC + 2 * c;
+        float lo, hi;
+        unpack(t[a][c], lo, hi);
+        A.store(at * S, lo);
+        A.store((at + 1) * S, hi);
+      }
     __syncthreads();
+  }
+  // Publishes the pivot rows and columns of tile column c (and c + 1) of grid column blk.
+  template <int TR, int TC>
+  __device__ __forceinline__ void publish_step(const uint64_t (&t)[TR][TC / 2], uint32_t row, uint32_t col, int pr, int pc,
+                                               int blk, int c) const {
+    constexpr int F = lane_grid_rows(P) / lane_grid_cols(P);
+    constexpr uint32_t kRow = (TR * lane_grid_rows(P) + 4) * S * 4;
+    if (pr == blk * F + c / TR) store_row<TC>(row, t[c % TR]);
+    if (pr == blk * F + (c + 1) / TR) store_row<TC>(row + kRow, t[(c + 1) % TR]);
+    if (pc == blk) {
+      float lo[TR], hi[TR];
+#pragma unroll
+      for (int a = 0; a < TR; ++a) unpack(t[a][c / 2], lo[a], hi[a]);
+      store_col<TR>(col, lo);
+      store_col<TR>(col + kRow, hi);
+    }
+  }
+  static __device__ __forceinline__ uint64_t pack(float lo, float hi) {
+    uint64_t v;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(lo), "f"(hi));
+    return v;
+  }
+  static __device__ __forceinline__ void unpack(uint64_t v, float& lo, float& hi) {
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+  }
+  static __device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+    uint64_t v;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(v) : "l"(a), "l"(b), "l"(c));
+    return v;
+  }
+  static __device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
+    uint64_t v;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(v) : "l"(a), "l"(b));
+    return v;
+  }
+  static __device__ __forceinline__ void load_pair(uint32_t at, float& a, float& b) {
+    asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(a), "=f"(b) : "r"(at));
+  }
+  template <int N>
+  static __device__ __forceinline__ void load_row(uint32_t at, uint64_t (&v)[N / 2]) {
+    if constexpr (N % 4 == 0) {
+#pragma unroll
+      for (int i = 0; i < N / 2; i += 2)
+        asm volatile("ld.shared.v2.u64 {%0, %1}, [%2];" : "=l"(v[i]), "=l"(v[i + 1]) : "r"(at + 8 * i));
+    } else {
+#pragma unroll
+      for (int i = 0; i < N / 2; ++i) asm volatile("ld.shared.u64 %0, [%1];" : "=l"(v[i]) : "r"(at + 8 * i));
+    }
+  }
+  template <int N>
+  static __device__ __forceinline__ void store_row(uint32_t at, const uint64_t (&v)[N / 2]) {
+    if constexpr (N % 4 == 0) {
+#pragma unroll
+      for (int i = 0; i < N / 2; i += 2)
+        asm volatile("st.shared.v2.u64 [%0], {%1, %2};" ::"r"(at + 8 * i), "l"(v[i]), "l"(v[i + 1]) : "memory");
+    } else {
+#pragma unroll
+      for (int i = 0; i < N / 2; ++i) asm volatile("st.shared.u64 [%0], %1;" ::"r"(at + 8 * i), "l"(v[i]) : "memory");
+    }
+  }
+  template <int N>
+  static __device__ __forceinline__ void load_col(uint32_t at, float (&v)[N]) {
+    if constexpr (N % 4 == 0) {
+#pragma unroll
+      for (int i = 0; i < N; i += 4)
+        asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
+                     : "=f"(v[i]), "=f"(v[i + 1]), "=f"(v[i + 2]), "=f"(v[i + 3])
+                     : "r"(at + 4 * i));
+    } else if constexpr (N % 2 == 0) {
+#pragma unroll
+      for (int i = 0; i < N; i += 2) load_pair(at + 4 * i, v[i], v[i + 1]);
+    } else {
+#pragma unroll
+      for (int i = 0; i < N; ++i) asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v[i]) : "r"(at + 4 * i));
+    }
+  }
+  template <int N>
+  static __device__ __forceinline__ void store_col(uint32_t at, const float (&v)[N]) {
+    if constexpr (N % 4 == 0) {
+#pragma unroll
+      for (int i = 0; i < N; i += 4)
+        asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(at + 4 * i), "f"(v[i]), "f"(v[i + 1]),
+                     "f"(v[i + 2]), "f"(v[i + 3])
+                     : "memory");
+    } else if constexpr (N % 2 == 0) {
+#pragma unroll
+      for (int i = 0; i < N; i += 2)
+        asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(at + 4 * i), "f"(v[i]), "f"(v[i + 1]) : "memory");
+    } else {
+#pragma unroll
+      for (int i = 0; i < N; ++i) asm volatile("st.shared.f32 [%0], %1;" ::"r"(at + 4 * i), "f"(v[i]) : "memory");
+    }
   }
 
   // The tail of the factorization, where there is one.
@@ -455,10 +555,10 @@ struct Kernel {
     if constexpr (kRefine) {
       switch (K.p.n_t / lane_grid_rows(P)) {
         case 0: break;
-        case lane_tile(P, 0): invert_tail<lane_tile(P, 0)>(); break;
-        case lane_tile(P, 1): invert_tail<lane_tile(P, 1)>(); break;
-        case lane_tile(P, 2): invert_tail<lane_tile(P, 2)>(); break;
-        default: invert_tail<lane_tile(P, 3)>(); break;
+        case lane_tile(P, W, 0): invert_tail<lane_tile(P, W, 0)>(); break;
+        case lane_tile(P, W, 1): invert_tail<lane_tile(P, W, 1)>(); break;
+        case lane_tile(P, W, 2): invert_tail<lane_tile(P, W, 2)>(); break;
+        default: invert_tail<lane_tile(P, W, 3)>(); break;
       }
     }
   }
@@ -469,7 +569,7 @@ struct Kernel {
       const int n = K.p.n_t;
       if (n == 0) return;
       const Shared<T> z{lus().at + (K.p.vec + K.p.ms) * S * static_cast<uint32_t>(sizeof(T))};
-      constexpr int NR = (lane_tile(P, 3) * lane_grid_rows(P) + P - 1) / P;
+      constexpr int NR = (lane_tile(P, W, 3) * lane_grid_rows(P) + P - 1) / P;
       T out[NR];
 #pragma unroll
       for (int a = 0; a < NR; ++a) {

@@ -341,8 +341,8 @@ int lane_tail_size(const LaneInput& in, const LanePattern& pat, const LaneShape&
   int best = 0;
   double best_cost = 0.0;
   for (int c = -1; c < kLaneTiles; ++c) {
-    const int tr = c < 0 ? 0 : lane_tile(P, c), n_t = tr * gr, tc = n_t / gc, ms = std::max(0, m - n_t);
-    if (c > 0 && lane_tile(P, c - 1) * gr >= m) break;  // the smaller tail already holds everything
+    const int tr = c < 0 ? 0 : lane_tile(P, warps, c), n_t = tr * gr, tc = n_t / gc, ms = std::max(0, m - n_t);
+    if (c > 0 && lane_tile(P, warps, c - 1) * gr >= m) break;  // the smaller tail already holds everything
     long n_ops = 0, n_lv = 0, nnz = 0;
     for (int k = 0; k < ms; ++k) {
       n_ops += ops[k];

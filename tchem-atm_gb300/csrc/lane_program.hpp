@@ -72,13 +72,12 @@ TCHEM_GB_HD constexpr int lane_grid_cols(int P) { return P >= 256 ? 16 : (P >= 6
 // two-way at most, and the padding could cost the second CTA per SM).
 TCHEM_GB_HD constexpr int lane_tail_stride(int P, int n_t) { return P > 16 ? n_t | 1 : n_t; }
 TCHEM_GB_HD constexpr int lane_grid_rows(int P) { return P / lane_grid_cols(P); }
-// Tile heights (rows per slot) that the kernel has for a slot count: n_t = height x grid rows.
+// Tile heights (rows per slot) that the kernel has for a slot count: n_t = height x grid rows. Widths are
+// even: the kernel takes pivots in pairs.
 constexpr int kLaneTiles = 4;
-TCHEM_GB_HD constexpr int lane_tile(int P, int k) {
-  return P >= 256 ? (k == 0 ? 2 : k == 1 ? 4 : k == 2 ? 7 : 10)
-                  : P >= 128 ? k + 1
-                  : P >= 64 ? (k == 0 ? 2 : k == 1 ? 3 : k == 2 ? 4 : 8)
-                  : P >= 32 ? k + 1 : (k == 0 ? 2 : k == 1 ? 4 : k == 2 ? 6 : 7);
+TCHEM_GB_HD constexpr int lane_tile(int P, int warps, int k) {
+  return P >= 256 ? (k == 0 ? 2 : k == 1 ? 4 : k == 2 || warps > 8 ? 8 : 10)  // 10 x 10 takes over 128 registers
+                  : P >= 128 ? k + 1 : P >= 64 ? 2 * (k + 1) : P >= 32 ? k + 1 : 2 * (k < 2 ? k + 1 : 3);
 }
 
 // Packets of each warp in turn, [rounds of the warp][slots per warp], and for the scheduled streams

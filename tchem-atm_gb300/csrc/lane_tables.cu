@@ -168,9 +168,9 @@ LaneTables* upload_aero_lane_tables(const HostTables& ht, const AeroDev& A, cons
 // The batched sparse-LU kernel's shape for a batch: the fewest samples per CTA (the most slots per
 // sample, the shortest round) that still hold the batch at once, else the most that one CTA per SM holds
 // (samples then follow each other through the lanes). The shape with two CTAs per SM takes longer per
-// round (51 species: 160 k cycles for 32 samples against 103 k for 16) and less per sample, so it pays
-// when its lanes are filled several times over: from twice its room (5,003 samples over 60 s: 556 ms
-// with one CTA per SM, 618 ms with two).
+// round (51 species: 160 k cycles for 32 samples against 104 k for 16) and less per sample, so it pays
+// when its lanes are filled several times over, from four times its room: 10,000 samples over 1 s 464 ms
+// with one CTA per SM, 494 ms with two; 16,384 695 and 690 ms; 40,000 1,462 and 1,343 ms.
 LanePlan plan_lanes(const LaneTables* t, LaneForm form, int ext, int sm_count, int max_smem, int nbatch) {
   LanePlan p;
   p.form = form;
@@ -179,7 +179,7 @@ LanePlan plan_lanes(const LaneTables* t, LaneForm form, int ext, int sm_count, i
     if (!t->valid[form][k]) continue;
     const LaneShape sh = kLaneShapes[k];
     const long room = static_cast<long>(sm_count) * sh.ctas * sh.S;
-    if (room <= best || (sh.ctas > 1 && nbatch < 2 * room && p.shape >= 0)) continue;
+    if (room <= best || (sh.ctas > 1 && nbatch < 4 * room && p.shape >= 0)) continue;
     best = room;
     p.shape = k;
     if (room >= nbatch) break;

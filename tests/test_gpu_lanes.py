@@ -61,7 +61,7 @@ def tadv_of(B, horizon, **kw):
 # one sample per CTA, two, four, eight, sixteen with one and with two CTAs per SM (152 SMs): a full
 # shape, one sample more, and odd remainders
 @pytest.mark.parametrize("form", ["mixed", "plain"])
-@pytest.mark.parametrize("B", [1, 152, 153, 305, 609, 1217, 2433, 9731])
+@pytest.mark.parametrize("B", [1, 152, 153, 305, 609, 1217, 2433, 19459])
 def test_every_shape_on_ragged_batches(B, form):
     km = KineticModel.from_string(mechanism_yaml(MechanismSpec()))
     state = sample_states(B, km.n_active, seed=B)
