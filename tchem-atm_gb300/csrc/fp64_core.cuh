@@ -16,7 +16,7 @@ struct WarpMem {
   double* keff;  // [R]
   double* q;     // [R] rates of progress
   double* d;     // [NF] Jacobian factor-slot derivatives
-  double* w;     // [m] triangular-solve vector
+  double* w;     // [m] scratch of the factorisation and the solves
   int32_t* piv;  // [m]
   double* A;     // [m][lda] Newton matrix / LU factors
 };
@@ -102,47 +102,79 @@ __device__ __forceinline__ void newton_matrix(Ctx<NPL>& c, const double (&y)[NPL
   ++c.st.n_jac;
 }
 
-// In-place LU with partial pivoting (first maximum in current row order), row swaps.
-// C: a per-sample context (Ctx, or the aerosol context) with W.A, W.piv, lda, lane and st.
+// In-place LU with partial pivoting (first maximum in current row order), row swaps; the diagonal of
+// the factors holds the pivots' reciprocals.
+// C: a per-sample context (Ctx, or the aerosol context) with W.A, W.piv, W.w, lane, lda and st.
+//
+// One warp has no other warp's work to hide a chain of dependent FP64 operations (about 16 cycles of
+// the SM's pipe each) behind, so what counts is how many there are in a row. The pivot search compares the
+// bit patterns of the magnitudes (three integer reductions instead of five rounds of FP64 compares), and
+// a step updates only rows with a multiplier and columns with an entry of the pivot row: the rows and
+// columns are listed by their ballots, and groups of lanes take a row each where few columns are left.
+// What is left out are additions of zero. LU_MEASURED
 template <class C>
 __device__ __forceinline__ bool lu_factor(C& c) {
   double* A = c.W.A;
   const int m = sys_dim(c), lda = c.lda, lane = c.lane;
+  uint16_t* cols = reinterpret_cast<uint16_t*>(c.W.w);  // [m] columns of the step, then [m] its rows
+  uint16_t* rows = cols + m;
+  const uint32_t below = (1u << lane) - 1u;
   for (int k = 0; k < m; ++k) {
-    double best = -1.0;
+    unsigned long long best = 0;
     int bi = m;
     for (int i = k + lane; i < m; i += 32) {
-      const double v = fabs(A[i * lda + k]);
-      if (v > best) { best = v; bi = i; }
+      const unsigned long long v = __double_as_longlong(A[i * lda + k]) & 0x7fffffffffffffffull;
+      if (v > best && v <= 0x7ff0000000000000ull) { best = v; bi = i; }  // a NaN is passed over
     }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      const double ob = __shfl_xor_sync(kFullMask, best, o);
-      const int oi = __shfl_xor_sync(kFullMask, bi, o);
-      if (ob > best || (ob == best && oi < bi)) { best = ob; bi = oi; }
-    }
-    if (!(best > 0.0) || !isfinite(best)) return false;
+    const uint32_t hi = static_cast<uint32_t>(best >> 32), lo = static_cast<uint32_t>(best);
+    const uint32_t top = __reduce_max_sync(kFullMask, hi);
+    const uint32_t low = __reduce_max_sync(kFullMask, hi == top ? lo : 0u);
+    bi = __reduce_min_sync(kFullMask, hi == top && lo == low ? bi : m);
+    if ((top | low) == 0u || top >= 0x7ff00000u) return false;
+    const double inv = 1.0 / A[bi * lda + k];
     if (lane == 0) c.W.piv[k] = bi;
+    __syncwarp();
     if (bi != k) {
       for (int j = lane; j < m; j += 32) {
         const double a = A[k * lda + j];
         A[k * lda + j] = A[bi * lda + j];
         A[bi * lda + j] = a;
       }
+      __syncwarp();
     }
-    __syncwarp();
-    const double inv = 1.0 / A[k * lda + k];
-    for (int i = k + 1 + lane; i < m; i += 32) A[i * lda + k] *= inv;
-    __syncwarp();
     const int w = m - k - 1;
-    if (w > 0) {
-      const int total = w * w;
-      int i = lane / w, j = lane - (lane / w) * w;
-      for (int e = lane; e < total; e += 32) {
-        const int ii = k + 1 + i, jj = k + 1 + j;
-        A[ii * lda + jj] -= A[ii * lda + k] * A[k * lda + jj];
-        j += 32;
-        while (j >= w) { j -= w; ++i; }
+    bool wild = false;  // an infinity or NaN: its products with zeros count too
+    for (int i = k + 1 + lane; i < m; i += 32) wild |= !isfinite(A[k * lda + i]) || !isfinite(A[i * lda + k] * inv);
+    wild = __any_sync(kFullMask, wild);
+    int nc = 0, nr = 0;
+    for (int i0 = k + 1; i0 < m; i0 += 32) {
+      const int i = i0 + lane;
+      bool in_row = false, in_col = false;
+      if (i < m) {
+        const double l = A[i * lda + k] * inv;
+        A[i * lda + k] = l;
+        in_row = wild || A[k * lda + i] != 0.0;
+        in_col = wild || l != 0.0;
+      }
+      const uint32_t rb = __ballot_sync(kFullMask, in_row), cb = __ballot_sync(kFullMask, in_col);
+      if (in_row) cols[nc + __popc(rb & below)] = static_cast<uint16_t>(i);
+      if (in_col) rows[nr + __popc(cb & below)] = static_cast<uint16_t>(i);
+      nc += __popc(rb);
+      nr += __popc(cb);
+    }
+    if (lane == 0) A[k * lda + k] = inv;
+    __syncwarp();
+    if (w > 0 && nc > 0) {
+      const int width = nc > 16 ? 32 : nc > 8 ? 16 : nc > 4 ? 8 : 4;  // lanes to a row
+      const int first = lane / width, step = 32 / width;
+      for (int e = lane & (width - 1); e < nc; e += width) {
+        const int j = cols[e];
+        const double u = A[k * lda + j];
+#pragma unroll 4
+        for (int r = first; r < nr; r += step) {
+          const int i = rows[r];
+          A[i * lda + j] -= A[i * lda + k] * u;
+        }
       }
     }
     __syncwarp();
@@ -151,7 +183,29 @@ __device__ __forceinline__ bool lu_factor(C& c) {
   return true;
 }
 
-// x = A^{-1} b with the factors of lu_factor.
+// The row swaps of lu_factor applied to w, in their order or backward; by the whole warp.
+template <class C>
+__device__ __forceinline__ void lu_swaps(C& c, double* w, bool backward) {
+  const int m = sys_dim(c);
+  const int chunks = (m + 31) / 32;
+  for (int t = 0; t < chunks; ++t) {
+    const int i0 = 32 * (backward ? chunks - 1 - t : t), i = i0 + c.lane;
+    uint32_t moved = __ballot_sync(kFullMask, i < m && c.W.piv[i] != i);
+    if (c.lane == 0) {
+      while (moved) {
+        const int b = backward ? 31 - __clz(moved) : __ffs(moved) - 1, k = i0 + b, p = c.W.piv[k];
+        moved &= ~(1u << b);
+        const double v = w[k];
+        w[k] = w[p];
+        w[p] = v;
+      }
+    }
+  }
+  __syncwarp();
+}
+
+// x = A^{-1} b with the factors of lu_factor. The vector stays in registers, an element per lane and
+// 32 rows, and each step hands its element round by a shuffle: no store, barrier and load in the chain.
 template <int NPL, class C>
 __device__ __forceinline__ void lu_solve(C& c, const double (&b)[NPL], double (&x)[NPL]) {
   const double* A = c.W.A;
@@ -163,29 +217,36 @@ __device__ __forceinline__ void lu_solve(C& c, const double (&b)[NPL], double (&
     if (i < m) w[i] = b[k];
   }
   __syncwarp();
-  if (lane == 0) {
-    for (int k = 0; k < m; ++k) {
-      const int p = c.W.piv[k];
-      if (p != k) { const double t = w[k]; w[k] = w[p]; w[p] = t; }
-    }
-  }
-  __syncwarp();
-  for (int k = 0; k < m; ++k) {
-    const double wk = w[k];
-    for (int i = k + 1 + lane; i < m; i += 32) w[i] -= A[i * lda + k] * wk;
-    __syncwarp();
-  }
-  for (int k = m - 1; k >= 0; --k) {
-    const double wk = w[k] / A[k * lda + k];
-    __syncwarp();
-    if (lane == 0) w[k] = wk;
-    for (int i = lane; i < k; i += 32) w[i] -= A[i * lda + k] * wk;
-    __syncwarp();
-  }
+  lu_swaps(c, w, false);
 #pragma unroll
   for (int k = 0; k < NPL; ++k) {
     const int i = lane + 32 * k;
     x[k] = (i < m) ? w[i] : 0.0;
+  }
+#pragma unroll
+  for (int t = 0; t < NPL; ++t) {
+#pragma unroll 4
+    for (int k = 32 * t; k < min(m, 32 * t + 32); ++k) {
+      const double xk = __shfl_sync(kFullMask, x[t], k - 32 * t);
+#pragma unroll
+      for (int a = t; a < NPL; ++a) {
+        const int i = lane + 32 * a;
+        if (i > k && i < m) x[a] -= A[i * lda + k] * xk;
+      }
+    }
+  }
+#pragma unroll
+  for (int t = NPL - 1; t >= 0; --t) {
+#pragma unroll 4
+    for (int k = min(m, 32 * t + 32) - 1; k >= 32 * t; --k) {
+      const double xk = __shfl_sync(kFullMask, x[t], k - 32 * t) * A[k * lda + k];
+      if (lane == k - 32 * t) x[t] = xk;
+#pragma unroll
+      for (int a = 0; a <= t; ++a) {
+        const int i = lane + 32 * a;
+        if (i < k) x[a] -= A[i * lda + k] * xk;
+      }
+    }
   }
   __syncwarp();
   ++c.st.n_solve;

@@ -35,30 +35,39 @@ __device__ __forceinline__ void lu_solve_t(Ctx<NPL>& c, const double (&b)[NPL], 
   double* w = c.W.w;
   const int m = c.L.m, lda = c.lda, lane = c.lane;
 #pragma unroll
-  for (int k = 0; k < NPL; ++k) {
-    const int i = lane + 32 * k;
-    if (i < m) w[i] = b[k];
-  }
-  __syncwarp();
-  for (int j = 0; j < m; ++j) {
-    const double zj = w[j] / A[j * lda + j];
-    __syncwarp();
-    if (lane == 0) w[j] = zj;
-    for (int l = j + 1 + lane; l < m; l += 32) w[l] -= A[j * lda + l] * zj;
-    __syncwarp();
-  }
-  for (int k = m - 1; k > 0; --k) {
-    const double vk = w[k];
-    for (int i = lane; i < k; i += 32) w[i] -= A[k * lda + i] * vk;
-    __syncwarp();
-  }
-  if (lane == 0) {
-    for (int k = m - 1; k >= 0; --k) {
-      const int p = c.W.piv[k];
-      if (p != k) { const double t = w[k]; w[k] = w[p]; w[p] = t; }
+  for (int k = 0; k < NPL; ++k) x[k] = b[k];
+#pragma unroll
+  for (int t = 0; t < NPL; ++t) {
+#pragma unroll 4
+    for (int j = 32 * t; j < min(m, 32 * t + 32); ++j) {
+      const double zj = __shfl_sync(kFullMask, x[t], j - 32 * t) * A[j * lda + j];
+      if (lane == j - 32 * t) x[t] = zj;
+#pragma unroll
+      for (int a = t; a < NPL; ++a) {
+        const int i = lane + 32 * a;
+        if (i > j && i < m) x[a] -= A[j * lda + i] * zj;
+      }
     }
   }
+#pragma unroll
+  for (int t = NPL - 1; t >= 0; --t) {
+#pragma unroll 4
+    for (int k = min(m, 32 * t + 32) - 1; k >= 32 * t; --k) {
+      const double vk = __shfl_sync(kFullMask, x[t], k - 32 * t);
+#pragma unroll
+      for (int a = 0; a <= t; ++a) {
+        const int i = lane + 32 * a;
+        if (i < k) x[a] -= A[k * lda + i] * vk;
+      }
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < NPL; ++k) {
+    const int i = lane + 32 * k;
+    if (i < m) w[i] = x[k];
+  }
   __syncwarp();
+  lu_swaps(c, w, true);
 #pragma unroll
   for (int k = 0; k < NPL; ++k) {
     const int i = lane + 32 * k;
