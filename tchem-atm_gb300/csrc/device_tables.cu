@@ -387,6 +387,7 @@ DeviceTables* upload_tables(const HostTables& ht, int device) {
   const size_t o_conv = sec(sizeof(int32_t) * R);
   const size_t o_cfp = sec(sizeof(int32_t) * (R + 1));
   const size_t o_cfi = sec(sizeof(int32_t) * std::max<size_t>(1, ht.cf_idx.size()));
+  const size_t o_pos = sec(sizeof(int32_t) * L.m);
   const size_t o_rxs = sec(sizeof(int32_t) * ht.rx_sidx.size());
   const size_t o_rxnu = sec(sizeof(double) * ht.rx_nu.size());
   const size_t o_rxn = sec(sizeof(int32_t) * ht.rx_n.size());
@@ -404,6 +405,8 @@ DeviceTables* upload_tables(const HostTables& ht, int device) {
   std::memcpy(host.data() + o_conv, ht.conv_exp.data(), sizeof(int32_t) * R);
   std::memcpy(host.data() + o_cfp, ht.cf_ptr.data(), sizeof(int32_t) * (R + 1));
   if (!ht.cf_idx.empty()) std::memcpy(host.data() + o_cfi, ht.cf_idx.data(), sizeof(int32_t) * ht.cf_idx.size());
+  for (int32_t i = 0; i < L.m; ++i)
+    reinterpret_cast<int32_t*>(host.data() + o_pos)[i] = ht.slu.lay.m == L.m ? ht.slu.pos[i] : i;
   std::memcpy(host.data() + o_rxs, ht.rx_sidx.data(), sizeof(int32_t) * ht.rx_sidx.size());
   std::memcpy(host.data() + o_rxnu, ht.rx_nu.data(), sizeof(double) * ht.rx_nu.size());
   std::memcpy(host.data() + o_rxn, ht.rx_n.data(), sizeof(int32_t) * ht.rx_n.size());
@@ -443,6 +446,7 @@ DeviceTables* upload_tables(const HostTables& ht, int device) {
   t->dev.cf_ptr = reinterpret_cast<const int32_t*>(b + o_cfp);
   t->dev.cf_idx = reinterpret_cast<const int32_t*>(b + o_cfi);
   t->dev.conv_ppm = CONV_PPM;
+  t->dev.pos = reinterpret_cast<const int32_t*>(b + o_pos);
   t->dev.rx_sidx = reinterpret_cast<const int32_t*>(b + o_rxs);
   t->dev.rx_nu = reinterpret_cast<const double*>(b + o_rxnu);
   t->dev.rx_n = reinterpret_cast<const int32_t*>(b + o_rxn);

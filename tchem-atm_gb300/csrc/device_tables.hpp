@@ -64,6 +64,7 @@ struct MechDev {
   // Stoichiometry by reaction in the reference's layout (KineticModelNCAR_ConstData reacSidx,
   // reacNuki, reacNreac, reacNprod): read by the adjoint for nu_r . mu.
   const int32_t* rx_sidx;  // [R][rx_S]
+  const int32_t* pos;      // [m] row of each species in the dense FP64 Newton matrix: the sparse LU's order, else its own
   const double* rx_nu;     // [R][rx_S], reactants signed negative, products from rx_S / 2
   const int32_t* rx_n;     // [R][2]: number of reactants, products
   int32_t rx_S;

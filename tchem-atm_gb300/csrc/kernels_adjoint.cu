@@ -15,7 +15,10 @@
 //   lambda_n = -cn mu2 + (I + c J(y_n))^T mu1.
 // Within each segment the forward states y_n, y_g are recomputed from the checkpoint with the
 // recorded step sizes (the same Newton code and inputs, so the same values) into a per-warp
-// global buffer, then the segment is swept backward.
+// global buffer, then the segment is swept backward. What bounds it is the chain of one warp's FP64 instructions in
+// the factorisations (fp64_core.cuh), 8 to 14 of them a step: recording and gradient of 64 samples of 51 species over
+// 3e-4 s take 126 ms where a pivot search by FP64 compares, updates of whole rows and solves through shared
+// memory took 250. Fewer warps per SM for small batches changed nothing (64 samples 81 and 83 ms).
 #include "advance.hpp"
 #include "engine.cuh"
 #include "fp64_core.cuh"
@@ -35,7 +38,16 @@ __device__ __forceinline__ void lu_solve_t(Ctx<NPL>& c, const double (&b)[NPL], 
   double* w = c.W.w;
   const int m = c.L.m, lda = c.lda, lane = c.lane;
 #pragma unroll
-  for (int k = 0; k < NPL; ++k) x[k] = b[k];
+  for (int k = 0; k < NPL; ++k) {
+    const int i = lane + 32 * k;
+    if (i < m) w[place(c, i)] = b[k];
+  }
+  __syncwarp();
+#pragma unroll
+  for (int k = 0; k < NPL; ++k) {
+    const int i = lane + 32 * k;
+    x[k] = (i < m) ? w[i] : 0.0;
+  }
 #pragma unroll
   for (int t = 0; t < NPL; ++t) {
 #pragma unroll 4
@@ -71,7 +83,7 @@ __device__ __forceinline__ void lu_solve_t(Ctx<NPL>& c, const double (&b)[NPL], 
 #pragma unroll
   for (int k = 0; k < NPL; ++k) {
     const int i = lane + 32 * k;
-    x[k] = (i < m) ? w[i] : 0.0;
+    x[k] = (i < m) ? w[place(c, i)] : 0.0;
   }
   __syncwarp();
   ++c.st.n_solve;
@@ -87,12 +99,13 @@ __device__ __forceinline__ void matvec_t(Ctx<NPL>& c, const double* mu, double (
     const int j = c.lane + 32 * k;
     double a0 = 0.0, a1 = 0.0;
     if (j < m) {
+      const double* col = A + place(c, j);
       int i = 0;
       for (; i + 1 < m; i += 2) {
-        a0 += A[i * lda + j] * mu[i];
-        a1 += A[(i + 1) * lda + j] * mu[i + 1];
+        a0 += col[place(c, i) * lda] * mu[i];
+        a1 += col[place(c, i + 1) * lda] * mu[i + 1];
       }
-      if (i < m) a0 += A[i * lda + j] * mu[i];
+      if (i < m) a0 += col[place(c, i) * lda] * mu[i];
     }
     out[k] = a0 + a1;
   }
@@ -189,7 +202,7 @@ __global__ void __launch_bounds__(256, 1) adjoint_fp64_kernel(const __grid_const
     }
     for (int r = lane; r < L.R; r += 32) gk[r] = 0.0;
     __syncwarp();
-    Ctx<NPL> c{L, T, W, lane, P.lda, tchem_gb_sample_stats{}};
+    Ctx<NPL> c{L, T, W, lane, P.lda, P.mech.pos, tchem_gb_sample_stats{}};
     NewtonSettings ns{ta.max_num_newton_iterations, ta.jacobian_interval > 0 ? ta.jacobian_interval : 1,
                       P.tol_newton[0], P.tol_newton[1]};
     const double* tdt = P.tape_dt + static_cast<size_t>(s) * P.tape_cap;

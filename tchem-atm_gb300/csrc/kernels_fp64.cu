@@ -118,7 +118,7 @@ __global__ void __launch_bounds__(256, 1) trbdf2_fp64_kernel(const __grid_consta
       atol[k] = (i < m) ? P.tol_time[2 * i] : 1.0;
       rtol[k] = (i < m) ? P.tol_time[2 * i + 1] : 0.0;
     }
-    Ctx<NPL> c{L, T, W, lane, P.lda, tchem_gb_sample_stats{}};
+    Ctx<NPL> c{L, T, W, lane, P.lda, P.mech.pos, tchem_gb_sample_stats{}};
     NewtonSettings nset = ns;
     nset.max_newton = ta.max_num_newton_iterations;
     nset.jac_interval = ta.jacobian_interval > 0 ? ta.jacobian_interval : 1;
