@@ -62,7 +62,7 @@ ATOL, RTOL = 1e-12, 1e-6
 SEED = 7
 UNCAPPED = 10_000_000  # step budget of a call that runs every sample to its horizon
 # Form names of the C ABI's tchem_gb_form.
-FORM_DTYPE = {"plain": "f64", "mixed": "f64 state / f32 Gauss-Jordan inverse or LU + f64-residual refinement",
+FORM_DTYPE = {"plain": "f64", "mixed": "f64 state / f32 sparse LU + f64-residual refinement",
               "simplified": "f64 state / f32 Gauss-Jordan inverse"}
 # DRAM bytes per sample of the time-advance kernel, from one ncu capture of a 4096-sample case of
 # the same kernel (dram__bytes_read.sum + dram__bytes_write.sum over the launch, divided by the
@@ -78,7 +78,7 @@ def parse() -> argparse.Namespace:
     ap.add_argument("--warmup", type=int, default=5, help="untimed calls on a separate copy of the batch")
     ap.add_argument("--impl", choices=["engine", "reference"], default="engine")
     ap.add_argument("--form", choices=["simplified", "mixed", "plain"], default="mixed",
-                    help="mixed (default): full Newton with an FP32 Gauss-Jordan inverse or LU and FP64-residual "
+                    help="mixed (default): full Newton with an FP32 sparse LU and FP64-residual "
                          "refinement; simplified: simplified Newton on a carried FP32 inverse; plain: FP64 LU")
     ap.add_argument("--samples", type=int, default=1 << 20, help="samples per GPU (the workload is 1,048,576)")
     ap.add_argument("--plain-samples", type=int, default=16384, help="subsample for the plain FP64 form")
@@ -571,19 +571,18 @@ def aerosol_leg(B: int, cpu_seconds: float, dev, stream) -> dict:
                                        f"over samples on {cores} threads ({el:.2f} s)"}}
 
 
-# ---- 300-species mechanism: the tensor-core form ------------------------------------------------
+# ---- 300-species mechanism ------------------------------------------------------------------------
 
 LARGE_SPEC = dict(n_species=300, n_reactions=1000, seed=20251205)
 
 
 def large_leg(B: int, horizon: float, dev, stream) -> dict:
     """The seeded 300-species / 1000-reaction mechanism (the large dense-LU configuration: same rate
-    mix, at most 2 reactants and 4 products) in the tensor-core form (full Newton; FP32 Newton
-    matrix, blocked LU with TF32 tcgen05 trailing updates, FP64 refinement), B samples over
-    `horizon`; the first 4 end states against the FP64 oracle; and the plain FP64 form beside it on
-    152 samples (one sample per SM) over 1e-4 s (49 steps; the plain form's FP64 LU in global memory
-    is too slow for longer), with the tensor-core form on the same samples and horizon, for the rate
-    ratio."""
+    mix, at most 2 reactants and 4 products) in the full-Newton FP32 form (batched sparse LU, FP64
+    refinement; a sample that would need pivoting takes the blocked LU with TF32 tcgen05 trailing
+    updates), B samples over `horizon`; the first 4 end states against the FP64 oracle; and the plain
+    FP64 form beside it on 152 samples (one sample per SM) over 1e-4 s (49 steps), with the FP32 form
+    on the same samples and horizon, for the rate ratio."""
     import torch
     from oracle import Oracle
     from tchem_gb import AtmosphericChemistry, tadv_to_device, time_advance_array
@@ -620,11 +619,11 @@ def large_leg(B: int, horizon: float, dev, stream) -> dict:
     ms_tc, *_ = run("mixed", P, 1e-4)
     ms_pl, res_pl, bad_pl, *_ = run("plain", P, 1e-4)
     names = ["steps", "rejected", "newton_fail", "newton_iter", "factorizations", "solves", "rhs", "jacobians"]
-    return {"samples": B, "species": m, "reactions": km.nReac, "horizon_s": horizon, "form": "tensor-core full Newton",
+    return {"samples": B, "species": m, "reactions": km.nReac, "horizon_s": horizon, "form": "mixed",
             "ms": ms, "value": B / (ms * 1e-3), "unit": "samples/s", "failed_samples": bad,
             "work_per_sample": {k: float(v) for k, v in zip(names, work)},
             "accuracy_vs_fp64_oracle": {"samples": K, "max": float(err.max()), "bound": 1e-6},
-            "vs_plain_fp64": {"samples": P, "horizon_s": 1e-4, "tensor_core_ms": ms_tc, "plain_fp64_ms": ms_pl,
+            "vs_plain_fp64": {"samples": P, "horizon_s": 1e-4, "mixed_ms": ms_tc, "plain_fp64_ms": ms_pl,
                               "speedup": ms_pl / ms_tc, "plain_failed_samples": bad_pl}}
 
 

@@ -146,7 +146,7 @@ typedef struct tchem_gb_sample_stats {
   int32_t n_newton_iter; /* Newton iterations, both stages */
   int32_t n_lu;          /* LU factorizations */
   int32_t n_solve;       /* forward+backward solve pairs (Newton updates and error filter) */
-  int32_t n_rhs;         /* right-hand-side evaluations */
+  int32_t n_rhs;         /* right-hand-side evaluations of the algorithm (one at a converged stage may be reused) */
   int32_t n_jac;         /* Jacobian evaluations */
 } tchem_gb_sample_stats;
 
@@ -165,8 +165,8 @@ int tchem_gb_mech_e3sm_view(const tchem_gb_mech* mech, tchem_gb_e3sm_view* view)
 /* Copies species name i (truncated as the reference stores it) into buf. */
 int tchem_gb_mech_species_name(const tchem_gb_mech* mech, int i, char* buf, int buflen);
 /* The static-order sparse LU of the mechanism's Newton matrix (no counterpart in the reference,
- * whose Tines solve factors the dense matrix with partial pivoting): the elimination program the
- * full-Newton FP32 form's one-warp shape runs for 33 to 128 active species. info[12] receives
+ * whose Tines solve factors the dense matrix with partial pivoting), as an elimination program for
+ * inspection; the batched kernel runs its own schedule of such a factorization. info[12] receives
  * m, nnz (entries of the filled pattern), n_ops (trailing updates), prog_len and the offsets
  * (int32 units into prog) of diag[m], pos[m], lc_ptr[m+1], lc[], uc_ptr[m+1], uc[], up_ptr[m+1]
  * and up[2 n_ops]: pos[s] is the elimination position of species s; diag[k] the entry of (k, k);
@@ -224,14 +224,16 @@ int tchem_gb_aero_scenario_particles(const char* yaml_path, const tchem_gb_aero*
 
 /* Numerical form of the time advance. */
 enum tchem_gb_form {
-  TCHEM_GB_FORM_PLAIN_FP64 = 0, /* FP64 Newton LU: the parity form */
-  /* The reference's full Newton with FP32 linear algebra -- an LU (one warp per sample,
-     threads_per_sample = 32: dense with partial pivoting up to 32 species, the static-order sparse
-     LU of tchem_gb_mech_sparse_lu from 33 to 128) or a Gauss-Jordan inverse (two or four warps per
-     sample, threads_per_sample = 64 or 128) -- and one sweep of
-     iterative refinement per Newton solve (FP64 residual of the linear system with the FP64
-     Jacobian, FP32 correction); FP64 Newton residual, state and error control: follows the FP64
-     form's Newton iterates. */
+  /* FP64 Newton LU: the parity form. Samples run in the batched sparse-LU kernel (a static fill-reducing
+     order, multipliers bounded by 64); a sample whose factorization would need pivoting, and every sample
+     with a jacobian_interval above 1, runs in the dense kernel with partial pivoting, in the same call. */
+  TCHEM_GB_FORM_PLAIN_FP64 = 0,
+  /* The reference's full Newton with FP32 linear algebra and one sweep of iterative refinement per
+     Newton solve (FP64 residual of the linear system with the FP64 Jacobian, FP32 correction); FP64
+     Newton residual, state and error control: follows the FP64 form's Newton iterates. The linear
+     algebra is the batched sparse LU, samples left over as above (threads_per_sample = 0, or 32 from 33
+     species up), a dense LU with partial pivoting (32, up to 32 species) or a Gauss-Jordan inverse on
+     two or four warps per sample (64 or 128). */
   TCHEM_GB_FORM_MIXED = 1,
   /* Simplified Newton with an FP32 Gauss-Jordan inverse of I - c J: the inverse is carried from
      the previous step's error filter while c changed by at most 30% (else formed at the first
@@ -250,7 +252,8 @@ typedef struct tchem_gb_advance_opts {
   int32_t form;               /* tchem_gb_form */
   int32_t threads_per_sample; /* mixed forms: 32, 64 or 128 threads (1, 2 or 4 warps) per sample;
                                  0: the mechanism's tuned preference (tchem_gb_autotune), else the
-                                 narrowest kernel shape for its size */
+                                 batched sparse LU (full Newton) or the narrowest kernel shape for the
+                                 mechanism's size (simplified) */
   int32_t reserved[6];        /* zero */
 } tchem_gb_advance_opts;
 

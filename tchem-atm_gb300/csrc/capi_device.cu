@@ -219,6 +219,10 @@ Plan make_plan(const tchem_gb_mech* const* mechs, int n_mechs, int nbatch, bool 
     off += up256(sizeof(int32_t) * static_cast<size_t>(plan.groups.size()) * std::max(nbatch, 1));
   }
   const DeviceInfo info = device_info(dev);
+  auto lanes_of = [&](const GroupPlan& g) {
+    return plan_lanes(dts[g.mechs[0]]->lanes, o.form == TCHEM_GB_FORM_PLAIN_FP64 ? LANE_F64 : LANE_F32, 0,
+                      info.sm_count, info.max_smem_optin, nbatch);
+  };
   for (auto& g : plan.groups) {
     const bool mixed = o.form == TCHEM_GB_FORM_MIXED || o.form == TCHEM_GB_FORM_MIXED_SIMPLIFIED;
     if (mixed) g.dev = dts[g.mechs[0]]->dev_x;  // sliced-ELL tables
@@ -246,9 +250,7 @@ Plan make_plan(const tchem_gb_mech* const* mechs, int n_mechs, int nbatch, bool 
       g.gmat_elems_per_warp = tc_advance_matrix_floats();  // floats per CTA
       g.gmat_offset = off;
       off += up256(sizeof(float) * g.gmat_elems_per_warp * static_cast<size_t>(g.grid));
-      if (o.form == TCHEM_GB_FORM_MIXED || o.form == TCHEM_GB_FORM_MIXED_SIMPLIFIED)
-        g.lanes = plan_lanes(dts[g.mechs[0]]->lanes, o.form == TCHEM_GB_FORM_PLAIN_FP64 ? LANE_F64 : LANE_F32, 0,
-                             info.sm_count, info.max_smem_optin, nbatch);
+      g.lanes = lanes_of(g);
       continue;
     }
     if (mixed) {
@@ -267,8 +269,7 @@ Plan make_plan(const tchem_gb_mech* const* mechs, int n_mechs, int nbatch, bool 
       g.ml = mc.ml;
       g.matrix_in_smem = true;
       g.lda = L.m;
-      if (o.form == TCHEM_GB_FORM_MIXED && tps == 0) g.lanes = plan_lanes(dts[g.mechs[0]]->lanes, o.form == TCHEM_GB_FORM_PLAIN_FP64 ? LANE_F64 : LANE_F32, 0,
-                             info.sm_count, info.max_smem_optin, nbatch);
+      if (o.form == TCHEM_GB_FORM_MIXED && tps == 0) g.lanes = lanes_of(g);
       continue;
     }
     g.lda = L.m | 1;
@@ -295,8 +296,7 @@ Plan make_plan(const tchem_gb_mech* const* mechs, int n_mechs, int nbatch, bool 
       g.gmat_offset = off;
       off += up256(sizeof(double) * g.gmat_elems_per_warp * static_cast<size_t>(g.grid) * W);
     }
-    g.lanes = plan_lanes(dts[g.mechs[0]]->lanes, o.form == TCHEM_GB_FORM_PLAIN_FP64 ? LANE_F64 : LANE_F32, 0,
-                             info.sm_count, info.max_smem_optin, nbatch);
+    g.lanes = lanes_of(g);
   }
   plan.bytes = off;
   return plan;

@@ -14,7 +14,7 @@
 //   mu1 = (I - c J(y_g))^-T (cg mu2),              dL/dtheta += c (q(y_g) + q(y_n)) (nu^T mu1)
 //   lambda_n = -cn mu2 + (I + c J(y_n))^T mu1.
 // Within each segment the forward states y_n, y_g are recomputed from the checkpoint with the
-// recorded step sizes (the same Newton code and inputs, so the same values) into a per-warp
+// recorded step sizes (the same Newton iteration to the same tolerance) into a per-warp
 // global buffer, then the segment is swept backward. What bounds it is the chain of one warp's FP64 instructions in
 // the factorisations (fp64_core.cuh), 8 to 14 of them a step: recording and gradient of 64 samples of 51 species over
 // 3e-4 s take 126 ms where a pivot search by FP64 compares, updates of whole rows and solves through shared

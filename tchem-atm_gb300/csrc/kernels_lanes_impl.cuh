@@ -17,11 +17,13 @@
 // Why: the dense kernels spend 44 k (LU) to 140 k (Gauss-Jordan) products on a 51-species matrix whose
 // sparse factors need 7.8 k, and every index of a sparse factorization costs as much as its product when
 // one warp works on one sample. What bounds this one: chains of dependent shared-memory loads and FP64
-// instructions (2 per cycle and SM) between barriers, 34 k cycles per round with one sample on the SM,
-// 103 k with 16. Measured against the dense kernels (one GB300): 51 species, one sample over 60 s 92 to
-// 56 ms, 4,096 samples over 3,600 s 1.20 to 1.04 s (FP32), 300 samples over 0.1 s 1.01 to 0.20 s (FP64);
-// 120 species, 257 samples over 1 s 440 to 238 ms; 300 species, 24 samples over 1e-4 s 442 to 65 ms (the
-// blocked LU on tensor cores with the matrix in L2); E3SM, 2,000 columns over 1,800 s 117 to 8.6 ms (FP64).
+// instructions (2 lanes per cycle and SM) between barriers, 34 k cycles per round with one sample on the SM,
+// 104 k with 16. FP32 with 16 samples: solves 21 k, tail 24 k, sparse factorization 12 k, matrix 11 k,
+// right-hand side 9 k, residual product 10 k, error test and norms 16 k. Measured against the dense kernels
+// (one GB300): 51 species, one sample over 60 s 93 ms to 54 ms, 4,096 samples over 3,600 s 1.20 s to 1.03 s (FP32), 300 samples
+// over 0.1 s 1.02 s to 204 ms (FP64); 120 species, 257 samples over 1 s 438 ms to 228 ms; 300 species, 24 samples over
+// 1e-4 s 443 ms to 75 ms (the blocked LU on tensor cores with the matrix in L2); E3SM, 2,000 columns over 1,800 s
+// 118 ms to 8.5 ms (FP64).
 //
 // T = float: the full-Newton FP32 form (FP32 matrix, factors and solves, FP64 residual, one
 // refinement sweep with an FP64 Jacobian-vector product per solve). T = double: the plain form.

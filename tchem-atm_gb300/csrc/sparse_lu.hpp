@@ -1,16 +1,14 @@
-// Static-order sparse LU of the Newton matrix I - c J (the sparse-LU shape of the full-Newton FP32
-// form, kernels_mixed_impl.cuh).
+// Static-order sparse LU of the Newton matrix I - c J as an elimination program for inspection
+// (tchem_gb_mech_sparse_lu). Its order is also the one the dense one-warp FP64 factorisation uses
+// (fp64_core.cuh); the batched kernel schedules its own (lane_program.hpp).
 //
 // The reference factors the dense Newton matrix with partial pivoting inside Tines
 // (src/core/problems/TChem_Impl_AtmosphericChemistry.hpp:138-155). A chemistry Jacobian is sparse
 // (the 51-species / 156-reaction benchmark mechanism: 507 of 2,601 entries), so here the structure
 // is analysed once per mechanism: a greedy Markowitz order on the diagonal (the remaining species
 // with the smallest (row count - 1) x (column count - 1), ties to the lowest species index), the
-// fill of that elimination, and a program of index lists that a warp runs per factorization
-// without any pivot search. The matrix I - c J of a mass-conserving mechanism has a diagonal of
-// 1 + c x (loss rate) >= 1; the kernel still tests every pivot (zero or non-finite: the Newton solve
-// fails, as the dense form's does), and the FP64-residual refinement sweep of every solve absorbs
-// the FP32 rounding of the factors.
+// fill of that elimination, and a program of index lists for a factorization without any pivot
+// search. The matrix I - c J of a mass-conserving mechanism has a diagonal of 1 + c x (loss rate) >= 1.
 //
 // Entries of the filled pattern are numbered row-major in position order (position k holds
 // species order[k]). The program is one int32 array with sections (offsets in SparseLuLayout):
