@@ -64,11 +64,11 @@ UNCAPPED = 10_000_000  # step budget of a call that runs every sample to its hor
 # Form names of the C ABI's tchem_gb_form.
 FORM_DTYPE = {"plain": "f64", "mixed": "f64 state / f32 sparse LU + f64-residual refinement",
               "simplified": "f64 state / f32 Gauss-Jordan inverse"}
-# DRAM bytes per sample of the time-advance kernel, from one ncu capture of a 4096-sample case of
+# DRAM bytes per sample of the time-advance kernel, from one ncu capture of a 2,432-sample case of
 # the same kernel (dram__bytes_read.sum + dram__bytes_write.sum over the launch, divided by the
 # samples). The per-sample traffic (state, time-advance record and times read once, results written
 # once) does not depend on the horizon or on the batch size, so it scales by samples.
-NCU_DRAM_BYTES_PER_SAMPLE = {"mixed": 820480 / 1216}  # 1,216-sample capture of the two-warp Gauss-Jordan kernel
+NCU_DRAM_BYTES_PER_SAMPLE = {"mixed": 3994880 / 2432}  # 2,432-sample capture of the batched sparse-LU kernel
 
 
 def parse() -> argparse.Namespace:
@@ -95,7 +95,7 @@ def parse() -> argparse.Namespace:
     ap.add_argument("--e3sm-samples", type=int, default=65536,
                     help="samples of the E3SM leg (the reference's 80-column uci scenario tiled); 0 skips it")
     ap.add_argument("--large-samples", type=int, default=1216,
-                    help="samples of the 300-species / 1000-reaction leg in the tensor-core form (with the plain "
+                    help="samples of the 300-species / 1000-reaction leg in the FP32 form (with the plain "
                          "FP64 form beside it on 152 samples over 0.1 s); 0 skips it")
     ap.add_argument("--large-horizon", type=float, default=10.0, help="horizon of the 300-species leg (s)")
     ap.add_argument("--tc-lu-matrices", type=int, default=0,
@@ -879,7 +879,7 @@ def engine_arm(args, world: int, rank: int, local: int):
                      "kernel_ms": kernel_ms, "launches": K,
                      "peak_source": "FMA-chain probe measured in this run (libtchem_gb_probe.so); "
                                     "MEASURED_PEAKS.json has no FP64/FP32 figure",
-                     "traffic_source": "DRAM bytes per sample from one ncu capture of a 4096-sample case of this "
+                     "traffic_source": "DRAM bytes per sample from one ncu capture of a 2,432-sample case of this "
                                        "kernel, times the samples of one launch",
                      "fp32": {"achieved": ach32, "peak": peak32.value / 1e12,
                               "frac": ach32 / (peak32.value / 1e12)},

@@ -251,7 +251,7 @@ int tchem_gb_aero_time_advance(const tchem_gb_mech* mech, const tchem_gb_aero* a
     plan = make_aero_plan(t->dev.L, A, nbatch, dev, false);
     const DeviceInfo info = device_info(dev);
     lanes = plan_lanes(aero_lanes_for(aero, *mech->host_tables, A, dev), LANE_AERO, lane_aero_doubles(A), info.sm_count,
-                       info.max_smem_optin, nbatch);
+                       info.max_smem_optin, nbatch, 1);
   } catch (const std::bad_alloc&) {
     return fail(TCHEM_GB_ERR_NOMEM, std::string(who) + ": allocation failed");
   } catch (const std::exception& e) {

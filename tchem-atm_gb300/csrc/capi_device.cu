@@ -221,7 +221,8 @@ Plan make_plan(const tchem_gb_mech* const* mechs, int n_mechs, int nbatch, bool 
   const DeviceInfo info = device_info(dev);
   auto lanes_of = [&](const GroupPlan& g) {
     return plan_lanes(dts[g.mechs[0]]->lanes, o.form == TCHEM_GB_FORM_PLAIN_FP64 ? LANE_F64 : LANE_F32, 0,
-                      info.sm_count, info.max_smem_optin, nbatch);
+                      info.sm_count, info.max_smem_optin, nbatch,
+                      e3sm ? 1 : o.form == TCHEM_GB_FORM_PLAIN_FP64 || g.dev.L.m > 64 ? 3 : 2);
   };
   for (auto& g : plan.groups) {
     const bool mixed = o.form == TCHEM_GB_FORM_MIXED || o.form == TCHEM_GB_FORM_MIXED_SIMPLIFIED;

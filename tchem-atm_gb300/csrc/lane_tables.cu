@@ -166,12 +166,19 @@ LaneTables* upload_aero_lane_tables(const HostTables& ht, const AeroDev& A, cons
 }
 
 // The batched sparse-LU kernel's shape for a batch: the fewest samples per CTA (the most slots per
-// sample, the shortest round) that still hold the batch at once, else the most that one CTA per SM holds
-// (samples then follow each other through the lanes). The shape with two CTAs per SM takes longer per
+// sample, the shortest round) whose lanes hold the batch at once, or `slack` times over, else the most
+// that one CTA per SM holds (samples then follow each other through the lanes). Box samples differ in length, the
+// longest taking about twice the mean, and the longest one's rounds are shorter with fewer samples beside it:
+// FP32 with up to 64 species gains up to twice the room (51 species over 2 s: 1,893 samples 232 ms with
+// 16 per CTA and 217 with 8, 1,230 samples 219 and 154, 230 samples 104 with two and 92 with one; 310 samples 93 with
+// two and 100 with one), where a round's time depends on the samples in it more than that (FP64, larger matrices) up to
+// three times (51 species FP64, 900 samples 155 ms with four and 141 with two; 120 species, 400 samples 144 ms with
+// two and 131 with one). E3SM columns and aerosol cells are alike in length and are held at once (FP64, 1,300
+// columns over 600 s: 12 ms with 8, 8 with 16). The shape with two CTAs per SM takes longer per
 // round (51 species: 160 k cycles for 32 samples against 104 k for 16) and less per sample, so it pays
 // when its lanes are filled several times over, from four times its room: 10,000 samples over 1 s 464 ms
 // with one CTA per SM, 494 ms with two; 16,384 695 and 690 ms; 40,000 1,462 and 1,343 ms.
-LanePlan plan_lanes(const LaneTables* t, LaneForm form, int ext, int sm_count, int max_smem, int nbatch) {
+LanePlan plan_lanes(const LaneTables* t, LaneForm form, int ext, int sm_count, int max_smem, int nbatch, int slack) {
   LanePlan p;
   p.form = form;
   long best = 0;
@@ -182,7 +189,7 @@ LanePlan plan_lanes(const LaneTables* t, LaneForm form, int ext, int sm_count, i
     if (room <= best || (sh.ctas > 1 && nbatch < 4 * room && p.shape >= 0)) continue;
     best = room;
     p.shape = k;
-    if (room >= nbatch) break;
+    if (slack * room >= nbatch) break;
   }
   if (p.shape < 0) return p;
   const LaneShape sh = kLaneShapes[p.shape];

@@ -28,7 +28,7 @@ struct LanePlan {
   LaneSmem smem{};
   LaneDev dev{};
 };
-LanePlan plan_lanes(const LaneTables* t, LaneForm form, int ext, int sm_count, int max_smem, int nbatch);
+LanePlan plan_lanes(const LaneTables* t, LaneForm form, int ext, int sm_count, int max_smem, int nbatch, int slack);
 void destroy_lane_tables(LaneTables* t);
 
 }  // namespace tchem_gb
