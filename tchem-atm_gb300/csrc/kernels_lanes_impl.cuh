@@ -565,10 +565,12 @@ struct Kernel {
     }
   }
 
-  // The tail rows of the vector section times the tail's inverse.
+  // The tail rows of the vector section times the tail's inverse. Rows beyond the species (a tail larger than
+  // the matrix) are inputs of zero for the whole launch and are not written: a non-finite sample would leave NaNs
+  // there for every later sample of the lane.
   __device__ __forceinline__ void apply_tail() {
     if constexpr (kRefine) {
-      const int n = K.p.n_t;
+      const int n = K.p.n_t, rows = K.p.m - K.p.ms;
       if (n == 0) return;
       const Shared<T> z{lus().at + (K.p.vec + K.p.ms) * S * static_cast<uint32_t>(sizeof(T))};
       constexpr int NR = (lane_tile(P, W, 3) * lane_grid_rows(P) + P - 1) / P;
@@ -577,7 +579,7 @@ struct Kernel {
       for (int a = 0; a < NR; ++a) {
         const int i = slot + P * a;
         T s0 = T(0), s1 = T(0);
-        if (i < n) {
+        if (i < rows) {
           const Shared<T> row{lus().at + (K.p.tail + i * lane_tail_stride(P, n)) * S * static_cast<uint32_t>(sizeof(T))};
 #pragma unroll 4
           for (int j = 0; j < n; j += 2) {
@@ -591,7 +593,7 @@ struct Kernel {
       __syncthreads();
 #pragma unroll
       for (int a = 0; a < NR; ++a)
-        if (slot + P * a < n) z.store((slot + P * a) * S, out[a]);
+        if (slot + P * a < rows) z.store((slot + P * a) * S, out[a]);
       __syncthreads();
     }
   }
