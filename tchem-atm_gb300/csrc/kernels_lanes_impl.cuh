@@ -1224,7 +1224,17 @@ struct Kernel {
             if (has(k)) xs()[pos(k) * S] = yn[k];
           }
         }
-        __syncthreads();  // outputs written before the lane is given away
+        // outputs written before the lane is given away
+        const bool rejected = AERO ? __syncthreads_or(code == C_REJECT) != 0 : (__syncthreads(), false);
+        if constexpr (AERO) {
+          // the transfers' terms are those of the rejected state; the matrix wants them at y_n again (the others'
+          // come out as they were, and q is free)
+          if (rejected) {
+            aero_particles();
+            __syncthreads();
+            aero_transfers();
+          }
+        }
         if (control && sl == 0 && code == C_DONE) {
           ci(I_CODE, s) = C_IDLE;
           ci(I_SMP, s) = -1;

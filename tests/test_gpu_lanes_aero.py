@@ -1,0 +1,56 @@
+"""The gas-aerosol problem in the batched sparse-LU kernel (csrc/kernels_lanes_impl.cuh) against the oracle: steps
+that follow a rejected one."""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+torch = pytest.importorskip("torch")
+
+from oracle import AerosolOracle  # noqa: E402
+from tchem_gb import _capi, tadv_to_device, time_advance_array  # noqa: E402
+from tchem_gb.aerosol import AerosolChemistry  # noqa: E402
+from test_zzz_gpu_aerosol import dev, models, perturbed  # noqa: E402
+
+pytestmark = pytest.mark.gpu
+
+TN = [1e-30, 1e-8]
+REDO_WORD = 192 // 4  # of the workspace: samples that the batched kernel left to the general one
+
+
+def advance(km, am, tadv, state, nc, tol):
+    """Results, work counters and the number of samples left to the general kernel."""
+    B = state.shape[0]
+    d_state = dev(state)
+    out, t = d_state.clone(), torch.zeros(B, dtype=torch.float64, device="cuda")
+    dt = torch.zeros_like(t)
+    ws = torch.zeros(AerosolChemistry.getWorkSpaceSize(km, am, B), dtype=torch.uint8, device="cuda")
+    stats = torch.zeros(B * _capi.SAMPLE_STATS_DTYPE.itemsize // 4, dtype=torch.int32, device="cuda")
+    status = AerosolChemistry.runDeviceBatch(dev(TN), dev(tol), None, tadv_to_device(tadv, torch.device("cuda")),
+                                             d_state, dev(nc), t, dt, out, km, am, stats=stats, workspace=ws)
+    torch.cuda.synchronize()
+    st = np.frombuffer(stats.cpu().numpy().tobytes(), dtype=_capi.SAMPLE_STATS_DTYPE)
+    return out.cpu().numpy(), t.cpu().numpy(), status.cpu().numpy(), st, int(ws.view(torch.int32)[REDO_WORD])
+
+
+# Few particles of 1e-18 to 1e-16 kg grow by orders of magnitude within a step, so the first attempts are rejected, and
+# the Newton test, on the norm of the gas, ends each stage after one iteration: what the matrix holds for the particles
+# goes straight into the result. Bound: the oracle's difference Jacobian is within 1e-8 of the exact one, over the twelve
+# attempts, with a factor 8 for what a step carries on.
+@pytest.mark.parametrize("rtol", [1e-4, 1e-6])
+def test_matrix_after_a_rejected_step(rtol):
+    km, am, gas, particles = models("simpol")
+    B, first = 16, 3 + km.nSpec
+    state, nc = perturbed(km, am, gas, particles, B, 2)
+    state[:, first:] = 10.0 ** np.random.default_rng(8).uniform(-18.0, -16.0, (B, state.shape[1] - first))
+    nc *= 1e-12
+    tadv = time_advance_array(B, tend=1000.0, dt=100.0, dtmin=1e-20, dtmax=1000.0, max_num_newton_iterations=20,
+                              num_time_iterations_per_interval=12)
+    tol = np.tile([1e-14, rtol], (am.n_ode, 1))
+    tol[km.n_active:, 0] = 1e-30
+    out, t, status, st, left = advance(km, am, tadv, state, nc, tol)
+    ref, t_ref, _, status_ref, st_ref = AerosolOracle(km, am).time_advance(tadv, state, nc, TN, tol)
+    assert left == 0 and np.array_equal(status, status_ref)
+    assert st_ref["n_rejected"].sum() > B and np.array_equal(st["n_rejected"], st_ref["n_rejected"])
+    assert (np.abs(t - t_ref) / t_ref).max() <= 1e-6
+    assert (np.abs(out[:, first:] - ref[:, first:]) / ref[:, first:]).max() <= 1e-6
