@@ -440,7 +440,9 @@ int tchem_gb_e3sm_time_advance(const tchem_gb_mech* mech, int nbatch, const doub
  * copied through. Refused with TCHEM_GB_ERR_UNSUPPORTED: a SIMPOL entry whose gas species is a
  * constant species, M above 320, or rate forms outside the box model's. The workspace holds the
  * work queue, the device error word (tchem_gb_device_error) and, for large M, the Newton
- * matrices: tchem_gb_aero_workspace_bytes (NULL workspace: library-owned). */
+ * matrices: tchem_gb_aero_workspace_bytes (NULL workspace: library-owned). That query, or an advance outside stream
+ * capture, also builds the batched kernel's tables for the model's particle count: a captured advance without them
+ * runs in the general kernel. */
 size_t tchem_gb_aero_workspace_bytes(const tchem_gb_mech* mech, const tchem_gb_aero* aero, int nbatch);
 int tchem_gb_aero_time_advance(const tchem_gb_mech* mech, const tchem_gb_aero* aero, int nbatch,
                                const double* tol_newton, const double* tol_time, const double* fac,

@@ -83,19 +83,30 @@ AeroDeviceTables* aero_tables_for(const tchem_gb_aero* aero, int dev) {
   return a->device_tables[dev];
 }
 
-// The batched kernel's streams for this mechanism and particle count (built on first use).
-const LaneTables* aero_lanes_for(const tchem_gb_aero* aero, const HostTables& ht, const AeroDev& A, int dev) {
+// The batched kernel's streams for this mechanism and particle count. Built by the workspace query or the first
+// advance, one entry per mechanism structure and particle count (at most kAeroMaxOde of them); without `build`, null
+// where there are none yet: an advance under capture must not allocate and runs in the general kernel.
+const LaneTables* aero_lanes_for(const tchem_gb_aero* aero, const HostTables& ht, const AeroDev& A, int dev,
+                                 bool build) {
   auto* a = const_cast<tchem_gb_aero*>(aero);
   std::lock_guard<std::mutex> lk(a->mu);
   AeroDeviceTables& t = *a->device_tables[dev];
   for (const AeroLanes& l : t.lanes)
     if (l.n_particles == A.nP && l.signature == ht.signature) return l.lanes;
+  if (!build) return nullptr;
   AeroLanes l;
   l.signature = ht.signature;
   l.n_particles = A.nP;
   l.lanes = upload_aero_lane_tables(ht, A, a->simpol_index.data(), dev, device_info(dev).max_smem_optin);
   t.lanes.push_back(l);
   return l.lanes;
+}
+
+bool under_capture(cudaStream_t stream) {
+  cudaStreamCaptureStatus c = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(stream, &c) == cudaSuccess) return c != cudaStreamCaptureStatusNone;
+  cudaGetLastError();  // the legacy stream beside another stream's capture
+  return true;
 }
 
 const HostTables* host_tables_of(const tchem_gb_mech* mech) {
@@ -217,6 +228,8 @@ size_t tchem_gb_aero_workspace_bytes(const tchem_gb_mech* mech, const tchem_gb_a
     int dev = 0;
     cudaGetDevice(&dev);
     const DeviceTables* t = tables_for(mech, dev);
+    fill_pointers(A, aero_tables_for(aero, dev));
+    aero_lanes_for(aero, *mech->host_tables, A, dev, true);
     return make_aero_plan(t->dev.L, A, nbatch, dev, false).bytes;
   } catch (const std::exception& e) {
     fail(TCHEM_GB_ERR_ARG, e.what());
@@ -250,8 +263,8 @@ int tchem_gb_aero_time_advance(const tchem_gb_mech* mech, const tchem_gb_aero* a
     fill_pointers(A, aero_tables_for(aero, dev));
     plan = make_aero_plan(t->dev.L, A, nbatch, dev, false);
     const DeviceInfo info = device_info(dev);
-    lanes = plan_lanes(aero_lanes_for(aero, *mech->host_tables, A, dev), LANE_AERO, lane_aero_doubles(A), info.sm_count,
-                       info.max_smem_optin, nbatch, 1);
+    lanes = plan_lanes(aero_lanes_for(aero, *mech->host_tables, A, dev, !under_capture(stream)), LANE_AERO,
+                       lane_aero_doubles(A), info.sm_count, info.max_smem_optin, nbatch, 1);
   } catch (const std::bad_alloc&) {
     return fail(TCHEM_GB_ERR_NOMEM, std::string(who) + ": allocation failed");
   } catch (const std::exception& e) {

@@ -1,5 +1,5 @@
 """The gas-aerosol problem in the batched sparse-LU kernel (csrc/kernels_lanes_impl.cuh) against the oracle: steps
-that follow a rejected one."""
+that follow a rejected one, and advances captured in a graph after the number of particles changed."""
 from __future__ import annotations
 
 import numpy as np
@@ -7,6 +7,7 @@ import pytest
 
 torch = pytest.importorskip("torch")
 
+from helpers import compare_tchem  # noqa: E402
 from oracle import AerosolOracle  # noqa: E402
 from tchem_gb import _capi, tadv_to_device, time_advance_array  # noqa: E402
 from tchem_gb.aerosol import AerosolChemistry  # noqa: E402
@@ -54,3 +55,35 @@ def test_matrix_after_a_rejected_step(rtol):
     assert st_ref["n_rejected"].sum() > B and np.array_equal(st["n_rejected"], st_ref["n_rejected"])
     assert (np.abs(t - t_ref) / t_ref).max() <= 1e-6
     assert (np.abs(out[:, first:] - ref[:, first:]) / ref[:, first:]).max() <= 1e-6
+
+
+@pytest.mark.parametrize("query", [True, False])
+def test_capture_after_a_change_of_particles(query):
+    km, am, gas, particles = models("simpol")
+    B = 5
+    state, nc = perturbed(km, am, gas, particles, B, 3)
+    tadv = time_advance_array(B, tend=1.0, dt=1e-6, dtmin=1e-20, dtmax=1.0, max_num_newton_iterations=20,
+                              num_time_iterations_per_interval=100000)
+    advance(km, am, tadv, state, nc, np.tile([1e-12, 1e-6], (am.n_ode, 1)))  # warm-up with one particle
+    ws_bytes = AerosolChemistry.getWorkSpaceSize(km, am, B)
+    am.set_number_of_particles(3)
+    if query:  # the query builds the new tables; without them the general kernel takes the call
+        ws_bytes = AerosolChemistry.getWorkSpaceSize(km, am, B)
+    state, nc = perturbed(km, am, gas, particles, B, 3)
+    tol = np.tile([1e-12, 1e-6], (am.n_ode, 1))
+    d = [dev(TN), dev(tol), None, tadv_to_device(tadv, torch.device("cuda")), dev(state), dev(nc)]
+    t, out = torch.zeros(B, dtype=torch.float64, device="cuda"), dev(state).clone()
+    dt, status = torch.zeros_like(t), torch.full((B,), -1, dtype=torch.int32, device="cuda")
+    ws = torch.zeros(ws_bytes, dtype=torch.uint8, device="cuda")
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        t.zero_()
+        AerosolChemistry.runDeviceBatch(*d, t, dt, out, km, am, status=status, workspace=ws)
+    ref = AerosolOracle(km, am).time_advance(tadv, state, nc, TN, tol)
+    for _ in range(2):
+        out.fill_(float("nan"))
+        graph.replay()
+        torch.cuda.synchronize()
+        assert np.array_equal(status.cpu().numpy(), ref[3]) and np.array_equal(t.cpu().numpy(), ref[1])
+        assert compare_tchem(out.cpu().numpy()[:, 3:], ref[0][:, 3:]) <= 1e-8
