@@ -231,9 +231,9 @@ enum tchem_gb_form {
   /* The reference's full Newton with FP32 linear algebra and one sweep of iterative refinement per
      Newton solve (FP64 residual of the linear system with the FP64 Jacobian, FP32 correction); FP64
      Newton residual, state and error control: follows the FP64 form's Newton iterates. The linear
-     algebra is the batched sparse LU, samples left over as above (threads_per_sample = 0, or 32 from 33
-     species up), a dense LU with partial pivoting (32, up to 32 species) or a Gauss-Jordan inverse on
-     two or four warps per sample (64 or 128). */
+     algebra is the batched sparse LU, samples left over as above (threads_per_sample = 0 as said at
+     tchem_gb_advance_opts, or 32 from 33 species up), a dense LU with partial pivoting (32, up to 32
+     species) or a Gauss-Jordan inverse on two or four warps per sample (64 or 128). */
   TCHEM_GB_FORM_MIXED = 1,
   /* Simplified Newton with an FP32 Gauss-Jordan inverse of I - c J: the inverse is carried from
      the previous step's error filter while c changed by at most 30% (else formed at the first
@@ -252,8 +252,9 @@ typedef struct tchem_gb_advance_opts {
   int32_t form;               /* tchem_gb_form */
   int32_t threads_per_sample; /* mixed forms: 32, 64 or 128 threads (1, 2 or 4 warps) per sample;
                                  0: the mechanism's tuned preference (tchem_gb_autotune), else the
-                                 batched sparse LU (full Newton) or the narrowest kernel shape for the
-                                 mechanism's size (simplified) */
+                                 batched sparse LU (full Newton; the narrowest kernel shape where that
+                                 is faster for the batch size: up to 64 species, below 128 samples per
+                                 SM) or the narrowest kernel shape for the mechanism's size (simplified) */
   int32_t reserved[6];        /* zero */
 } tchem_gb_advance_opts;
 

@@ -219,10 +219,11 @@ Plan make_plan(const tchem_gb_mech* const* mechs, int n_mechs, int nbatch, bool 
     off += up256(sizeof(int32_t) * static_cast<size_t>(plan.groups.size()) * std::max(nbatch, 1));
   }
   const DeviceInfo info = device_info(dev);
-  auto lanes_of = [&](const GroupPlan& g) {
-    return plan_lanes(dts[g.mechs[0]]->lanes, o.form == TCHEM_GB_FORM_PLAIN_FP64 ? LANE_F64 : LANE_F32, 0,
-                      info.sm_count, info.max_smem_optin, nbatch,
-                      e3sm ? 1 : o.form == TCHEM_GB_FORM_PLAIN_FP64 || g.dev.L.m > 64 ? 3 : 2);
+  auto lanes_of = [&](const GroupPlan& g, bool asked = false) {
+    const LaneForm form = o.form == TCHEM_GB_FORM_PLAIN_FP64 ? LANE_F64 : LANE_F32;
+    if (!asked && !e3sm && !lanes_pay_for_box(form, g.dev.L.m, info.sm_count, nbatch)) return LanePlan{};
+    return plan_lanes(dts[g.mechs[0]]->lanes, form, 0, info.sm_count, info.max_smem_optin, nbatch,
+                      e3sm ? 1 : form == LANE_F64 || g.dev.L.m > 64 ? 3 : 2);
   };
   for (auto& g : plan.groups) {
     const bool mixed = o.form == TCHEM_GB_FORM_MIXED || o.form == TCHEM_GB_FORM_MIXED_SIMPLIFIED;
@@ -259,7 +260,8 @@ Plan make_plan(const tchem_gb_mech* const* mechs, int n_mechs, int nbatch, bool 
       if (tps == 0 && o.form >= 0 && o.form < 3) tps = mechs[g.mechs[0]]->tps_pref[o.form];
       // full Newton, one warp's worth of threads above 32 species: the batched sparse-LU kernel (the
       // samples it leaves go to the Gauss-Jordan shape)
-      if (o.form == TCHEM_GB_FORM_MIXED && tps == 32 && L.m > 32 && L.m <= 128 && !e3sm) tps = 0;
+      const bool asked = o.form == TCHEM_GB_FORM_MIXED && tps == 32 && L.m > 32 && L.m <= 128 && !e3sm;
+      if (asked) tps = 0;
       MixedConfig mc = mixed_config(L, tps, info.sm_count, info.max_smem_optin, nbatch,
                                     o.form == TCHEM_GB_FORM_MIXED_SIMPLIFIED, e3sm);
       g.kernel = mc.kernel;
@@ -270,7 +272,7 @@ Plan make_plan(const tchem_gb_mech* const* mechs, int n_mechs, int nbatch, bool 
       g.ml = mc.ml;
       g.matrix_in_smem = true;
       g.lda = L.m;
-      if (o.form == TCHEM_GB_FORM_MIXED && tps == 0) g.lanes = lanes_of(g);
+      if (o.form == TCHEM_GB_FORM_MIXED && tps == 0) g.lanes = lanes_of(g, asked);
       continue;
     }
     g.lda = L.m | 1;

@@ -203,6 +203,29 @@ LanePlan plan_lanes(const LaneTables* t, LaneForm form, int ext, int sm_count, i
   return p;
 }
 
+// A round of the batched kernel has some 70 (FP32) to 175 (FP64) CTA barriers however small the matrix, which a
+// one-warp or two-warp kernel on a matrix in registers does not pay: few species, or so many samples that the SMs
+// hold that kernel's warps one beside the other, and the batched kernel is the slower one until the batch fills
+// its two-CTA shape (128 samples per SM). Measured on 152 SMs, ms of the register kernel / of the batched one:
+//  * FP32, up to 32 species (one warp, dense LU): 8 species over 1e-2 s, 150 samples 19.6 / 22.7, 1,000 22.5 / 29.9, 10,000
+//    44 / 50, 20,000 74 / 50; 20 species over 1e-2 s, 150 samples 32 / 23, 600 32 / 33, 4,000 42 / 62, 20,000 88 / 85;
+//    32 species over 1e-2 s, 1,000 samples 54 / 43, 2,000 63 / 60, 4,000 67 / 83, 20,000 146 / 135. The first crossing
+//    goes with the square of the species: at 1.2, 3.3 and 8.5 samples per SM for 12, 20 and 32 species.
+//  * FP32, 33 to 64 species (two warps, Gauss-Jordan): between 5.5 and 14 samples per SM. 51 species over 60 s, 800
+//    samples 234 / 227, 900 231 / 237, 1,600 322 / 333, 2,432 413 / 400; over 1e-3 s, 800 48 / 45, 1,250 47 / 53,
+//    1,900 55 / 58; 64 species over 1e-2 s, 900 samples 41 / 49, 1,900 48 / 56. Above it the batched kernel wins over
+//    seconds and more (51 species over 60 s, 4,000 samples 588 / 520) and loses where a few samples need many times
+//    the others' iterations (over 1e-3 s, 4,000 samples 62 / 68 to 87); the horizon is not known on the host.
+//  * FP64, up to 3 species: over 1e-3 s, 150 samples 1.14 / 0.83, 1,000 1.17 / 1.97, 2,000 2.1 / 2.0.
+bool lanes_pay_for_box(LaneForm form, int m, int sm_count, int nbatch) {
+  const long B = nbatch, sms = sm_count;
+  if (B >= 128 * sms) return true;
+  if (form != LANE_F32) return m > 3 || B <= sms || B > 13 * sms;
+  if (m <= 8) return false;
+  if (m <= 32) return 120 * B <= sms * m * m;
+  return m > 64 || 2 * B <= 11 * sms || B > 14 * sms;
+}
+
 void destroy_lane_tables(LaneTables* t) {
   if (!t) return;
   int prev = 0;

@@ -29,6 +29,9 @@ struct LanePlan {
   LaneDev dev{};
 };
 LanePlan plan_lanes(const LaneTables* t, LaneForm form, int ext, int sm_count, int max_smem, int nbatch, int slack);
+// Whether the batched kernel is the faster default for a box-model batch of mechanisms with m species (E3SM columns
+// and aerosol cells always take it).
+bool lanes_pay_for_box(LaneForm form, int m, int sm_count, int nbatch);
 void destroy_lane_tables(LaneTables* t);
 
 }  // namespace tchem_gb

@@ -1,7 +1,7 @@
 """Lanes of the batched sparse-LU time advance (csrc/kernels_lanes_impl.cuh) that held a sample with non-finite
 values and take another from the queue: the later samples come out as the oracle's. The batches are larger than
-the shapes' lanes, so that a lane is refilled, and the FP32 cases below 32 species have a tail block with more
-rows than the matrix (32, 16, 32 and 8 rows at one, eight, two and sixteen samples per CTA on 152 SMs).
+the shapes' lanes, so that a lane is refilled, and the last FP32 cases have a tail block with more rows than the
+matrix (32 rows at one and two samples per CTA and 8 rows at sixteen, on 152 SMs).
 Bounds are the forms' own: 1e-6 per species for the full-Newton FP32 form, 1e-8 for the plain form."""
 from __future__ import annotations
 
@@ -28,7 +28,8 @@ def dev(a):
 @pytest.mark.parametrize("form", ["mixed", "plain"])
 @pytest.mark.parametrize("bad", [np.nan, np.inf])
 @pytest.mark.parametrize("m,R,B,horizon", [(8, 20, 290, 1e-3), (4, 9, 2000, 1e-2), (20, 60, 580, 1e-3), (3, 5, 4500, 1.0),
-                                           (51, 156, 290, 1e-6)])
+                                           (51, 156, 290, 1e-6), (12, 36, 180, 1e-3), (20, 60, 500, 1e-3),
+                                           (4, 9, 19600, 1e-4)])
 def test_samples_after_a_non_finite_one(m, R, B, horizon, bad, form):
     km = KineticModel.from_string(mechanism_yaml(MechanismSpec(n_species=m, n_reactions=R, seed=1000 + m)))
     state = sample_states(B, m, seed=7)
