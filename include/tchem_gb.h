@@ -349,12 +349,14 @@ int tchem_gb_adjoint(const tchem_gb_mech* mech, int nbatch, const double* tol_ne
 
 /* Autotuner (no counterpart in the reference, whose team sizes are fixed at launch): times the
  * form's kernel shapes (32, 64 and 128 threads per sample, where a shape exists for the
- * mechanism's size) on a probe batch of device arrays laid out as for tchem_gb_time_advance
- * (t_out is zeroed before every trial: the probe starts at t = 0; workspace may be NULL), keeps the
- * fastest as the mechanism's preference for calls with opts.threads_per_sample == 0, and returns
- * it in *chosen; ms_per_candidate[3] (optional) receives each trial's time (-1: not run).
+ * mechanism's size) and the full-Newton form's default on a probe batch of device arrays laid out as for
+ * tchem_gb_time_advance (t_out is zeroed before every trial: the probe starts at t = 0; workspace may be NULL),
+ * keeps the fastest as the mechanism's preference for calls with opts.threads_per_sample == 0, and returns
+ * it in *chosen: 0 (no preference) where the full-Newton form's default, which goes by each batch's size, is
+ * within 3 % of the fastest. ms_per_candidate[3] (optional) receives the shapes' times (-1: not run).
+ * An E3SM advance of the full-Newton form takes its default whatever the preference.
  * Synchronizes the stream. tchem_gb_mech_set_threads_per_sample sets the preference directly
- * (0: the narrowest shape). */
+ * (0: none). */
 int tchem_gb_autotune(tchem_gb_mech* mech, int form, int nbatch, const double* tol_newton, const double* tol_time,
                       const tchem_gb_tadv* tadv, const double* state, double* t_out, double* dt_out,
                       double* state_out, int32_t* status, void* workspace, size_t workspace_bytes, void* stream,

@@ -178,8 +178,10 @@ struct Plan {
 // Groups structurally identical mechanisms and sizes each group's launch.
 // e3sm: the E3SM time advance (per-sample rate constants and source terms): every rate form of
 // the E3SM tables is allowed, and each warp group gets a source-term section.
+// use_pref: the mechanism's tuned preference stands in for threads_per_sample == 0. Not in the E3SM advance of the
+// full-Newton form: the preference is one between box-model kernels, of which E3SM has none but its default.
 Plan make_plan(const tchem_gb_mech* const* mechs, int n_mechs, int nbatch, bool have_mos, const tchem_gb_advance_opts& o,
-               int dev, bool e3sm = false) {
+               int dev, bool e3sm = false, bool use_pref = true) {
   if (n_mechs <= 0 || n_mechs > kMaxMechs) throw std::invalid_argument("n_mechs must be in [1, 64]");
   Plan plan;
   std::vector<const HostTables*> hts(n_mechs);
@@ -257,7 +259,7 @@ Plan make_plan(const tchem_gb_mech* const* mechs, int n_mechs, int nbatch, bool 
     }
     if (mixed) {
       int tps = o.threads_per_sample;
-      if (tps == 0 && o.form >= 0 && o.form < 3) tps = mechs[g.mechs[0]]->tps_pref[o.form];
+      if (tps == 0 && use_pref && !(e3sm && o.form == TCHEM_GB_FORM_MIXED)) tps = mechs[g.mechs[0]]->tps_pref[o.form];
       // full Newton, one warp's worth of threads above 32 species: the batched sparse-LU kernel (the
       // samples it leaves go to the Gauss-Jordan shape)
       const bool asked = o.form == TCHEM_GB_FORM_MIXED && tps == 32 && L.m > 32 && L.m <= 128 && !e3sm;
@@ -385,7 +387,7 @@ int time_advance_impl(const tchem_gb_mech* const* mechs, int n_mechs, const int3
                       const double* state, double* t_out, double* dt_out, double* state_out, int32_t* status,
                       tchem_gb_sample_stats* stats, void* workspace, size_t workspace_bytes,
                       const tchem_gb_advance_opts* opts, void* stream_v, const TapeArgs& tape,
-                      const RateArgs& rates = RateArgs{}) {
+                      const RateArgs& rates = RateArgs{}, bool use_pref = true) {
   if (!mechs || nbatch < 0) return fail(TCHEM_GB_ERR_ARG, "tchem_gb_time_advance: bad mechanisms or batch size");
   if (nbatch == 0) return TCHEM_GB_OK;  // empty arrays may come with null pointers
   if (!tol_newton || !tol_time || !tadv || !state || !t_out || !dt_out || !state_out || !status)
@@ -398,7 +400,7 @@ int time_advance_impl(const tchem_gb_mech* const* mechs, int n_mechs, const int3
   cudaGetDevice(&dev);
   Plan plan;
   try {
-    plan = make_plan(mechs, n_mechs, nbatch, mech_of_sample != nullptr, o, dev, rates.keff != nullptr);
+    plan = make_plan(mechs, n_mechs, nbatch, mech_of_sample != nullptr, o, dev, rates.keff != nullptr, use_pref);
     const int n0 = mechs[0]->km.nSpec;
     for (int i = 1; i < n_mechs; ++i)
       if (mechs[i]->km.nSpec + 3 > n0 + 3 && mech_of_sample == nullptr)
@@ -712,16 +714,20 @@ int tchem_gb_autotune(tchem_gb_mech* mech, int form, int nbatch, const double* t
                       int* chosen, float* ms_per_candidate) {
   if (!mech || form < 0 || form > 2 || nbatch <= 0 || !chosen)
     return fail(TCHEM_GB_ERR_ARG, "tchem_gb_autotune: bad argument");
-  const int cands[3] = {32, 64, 128};
+  // 0: the default of the full-Newton form, the batched kernel or the narrowest shape by the size of each batch. It
+  // stays (no preference) unless a shape beats it by more than the runs of one kernel differ.
+  const int cands[4] = {0, 32, 64, 128};
+  const float kClearly = 0.97f;
   cudaStream_t stream = static_cast<cudaStream_t>(stream_v);
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   if (cudaEventCreate(&e0) != cudaSuccess || cudaEventCreate(&e1) != cudaSuccess)
     return fail(TCHEM_GB_ERR_CUDA, "tchem_gb_autotune: cudaEventCreate failed");
   float best_ms = 0.f;
-  int best = 0;
+  int best = -1;
   const tchem_gb_mech* mechs[1] = {mech};
-  for (int c = 0; c < 3; ++c) {
-    if (ms_per_candidate) ms_per_candidate[c] = -1.f;
+  for (int c = 0; c < 4; ++c) {
+    if (ms_per_candidate && c > 0) ms_per_candidate[c - 1] = -1.f;
+    if (cands[c] == 0 && form != TCHEM_GB_FORM_MIXED) continue;
     tchem_gb_advance_opts o{};
     o.form = form;
     o.threads_per_sample = cands[c];
@@ -730,7 +736,8 @@ int tchem_gb_autotune(tchem_gb_mech* mech, int form, int nbatch, const double* t
     cudaMemsetAsync(t_out, 0, sizeof(double) * nbatch, stream);       // the probe starts at t = 0
     cudaEventRecord(e0, stream);
     const int rc = time_advance_impl(mechs, 1, nullptr, nbatch, tol_newton, tol_time, tadv, state, t_out, dt_out,
-                                     state_out, status, nullptr, workspace, workspace_bytes, &o, stream_v, TapeArgs{});
+                                     state_out, status, nullptr, workspace, workspace_bytes, &o, stream_v, TapeArgs{},
+                                     RateArgs{}, false);
     cudaEventRecord(e1, stream);
     if (rc != TCHEM_GB_OK) {
       cudaEventDestroy(e0);
@@ -744,15 +751,15 @@ int tchem_gb_autotune(tchem_gb_mech* mech, int form, int nbatch, const double* t
     }
     float ms = 0.f;
     cudaEventElapsedTime(&ms, e0, e1);
-    if (ms_per_candidate) ms_per_candidate[c] = ms;
-    if (best == 0 || ms < best_ms) {
+    if (ms_per_candidate && c > 0) ms_per_candidate[c - 1] = ms;
+    if (best < 0 || ms < best_ms * (best == 0 ? kClearly : 1.f)) {
       best = cands[c];
       best_ms = ms;
     }
   }
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
-  if (best == 0) return fail(TCHEM_GB_ERR_UNSUPPORTED, "tchem_gb_autotune: no kernel shape for this mechanism");
+  if (best < 0) return fail(TCHEM_GB_ERR_UNSUPPORTED, "tchem_gb_autotune: no kernel shape for this mechanism");
   {
     std::lock_guard<std::mutex> lk(mech->mu);
     mech->tps_pref[form] = best;

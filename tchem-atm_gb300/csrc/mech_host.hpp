@@ -33,7 +33,7 @@ struct tchem_gb_mech {
   std::vector<tchem_gb::DeviceTables*> device_tables;
   std::mutex mu;
   // Threads per sample used when a call leaves it to the library (opts.threads_per_sample == 0),
-  // per tchem_gb_form; 0: the narrowest kernel shape. Set by tchem_gb_autotune.
+  // per tchem_gb_form; 0: the form's default (threads_per_sample). Set by tchem_gb_autotune.
   int tps_pref[3] = {0, 0, 0};
 
   void build_view();

@@ -152,7 +152,8 @@ class AtmosphericChemistry:
                  stream=None):
         """Times the form's kernel shapes (32/64/128 threads per sample) on the probe batch (device
         arrays as for runDeviceBatch; the probe starts at t = 0), keeps the fastest as the mechanism's
-        default and returns (threads_per_sample, {shape: ms})."""
+        default and returns (threads_per_sample, {shape: ms}); 0 threads: the full-Newton form's own
+        default, which goes by each batch's size, is as fast as any (its time is not in the dict)."""
         torch = _torch()
         B = int(state.shape[0])
         out = torch.empty_like(state)
