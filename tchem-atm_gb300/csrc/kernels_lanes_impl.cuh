@@ -46,7 +46,8 @@ namespace lanes {
 
 // Largest multiplier |l_ik| accepted without pivoting. The diagonal of I - c J is 1 + c x (loss
 // rate), and a column's off-diagonal entries are c x (loss rate) x yield, so multipliers stay near
-// the yields (about 1); partial pivoting would bound them by 1.
+// the yields (about 1); partial pivoting would bound them by 1. Columns whose pivot row has no further entries are
+// not asked (lane_program.cpp).
 constexpr float kLaneMaxGrowth = 64.f;
 constexpr int kLaneMaxGrowthHi = 0x40500000;  // the high word of 64.0
 

@@ -521,6 +521,11 @@ LaneProgram build_lane_program(const LaneInput& in, const LanePattern& pat, int 
     return st;
   };
   {
+    // a pivot row without other entries is subtracted from no one: its column's multipliers only enter the substitution,
+    // whatever their size
+    std::vector<char> spreads(m, 0);
+    for (int k = 0; k < ms; ++k)
+      for (int l = k + 1; l < m; ++l) spreads[k] |= E(k, l) >= 0;
     std::vector<Task> tasks;
     for (int i = 0; i < m; ++i)
       for (int j = 0; j < m; ++j) {
@@ -534,7 +539,7 @@ LaneProgram build_lane_program(const LaneInput& in, const LanePattern& pat, int 
         if (i == j && i < ms) {
           t.flags = LP_PIVOT;
         } else if (i > j && j < ms) {
-          t.flags = LP_LCOL;
+          t.flags = spreads[j] ? uint32_t(LP_LCOL) : 0u;
           t.scale = j;
         } else if (t.ops.empty()) {
           continue;  // final as assembled

@@ -38,12 +38,13 @@ def left(ws, groups=1):
     return ws.view(torch.int32)[REDO_WORD:REDO_WORD + groups].cpu().tolist()
 
 
-# A -> 200 B, B -> C, C -> 0.001 A and a chain of nine more: the multiplier of A's column is near 200 for long steps
-def growth():
+# A -> 200 B, B -> C, C -> 0.001 A and a ring of nine more: the multiplier of A's column is near 200 for long steps.
+# Without the last of the three nothing but A itself is in A's row, which is then subtracted from no other.
+def growth(feedback=True):
     lines = ["NCAR-version: v1.0", "constant_species:", "- name: M", "species:"]
     names = ["A", "B", "C"] + [f"X{i}" for i in range(9)]
     lines += [f"- name: {n}" for n in names] + ["reactions:"]
-    steps = [("A", "B", 200, 1.0e3), ("B", "C", 1, 0.5), ("C", "A", 0.001, 0.1)]
+    steps = [("A", "B", 200, 1.0e3), ("B", "C", 1, 0.5), ("C", "A" if feedback else "X0", 0.001, 0.1)]
     steps += [(f"X{i}", f"X{(i + 1) % 9}", 1, 0.1 * (i + 1)) for i in range(9)]
     for a, b, n, k in steps:
         lines += ["- reactants:", f"    {a}: 1", "  products:", f"    {b}: {n}", "  type: ARRHENIUS", "  coefficients:",
@@ -52,8 +53,9 @@ def growth():
 
 
 @pytest.mark.parametrize("form", ["mixed", "plain"])
-def test_multipliers_beyond_the_bound_are_handed_over(form):
-    km, B = growth(), 19
+@pytest.mark.parametrize("feedback", [True, False])
+def test_multipliers_beyond_the_bound_are_handed_over(feedback, form):
+    km, B = growth(feedback), 19
     m = km.n_active
     state, tadv, tol = sample_states(B, m, seed=11), tadv_of(B, 50.0), np.tile([1e-12, 1e-6], (12, 1))
     ws = torch.zeros(AtmosphericChemistry.getWorkSpaceSize(km, B, form), dtype=torch.uint8, device="cuda")
@@ -62,7 +64,7 @@ def test_multipliers_beyond_the_bound_are_handed_over(form):
     st = AtmosphericChemistry.runDeviceBatch(dev(TN), dev(tol), None, tadv_to_device(tadv), d_state, t,
                                              torch.zeros_like(t), out, km, form=form, workspace=ws)
     ref = Oracle([km]).time_advance(tadv, state, TN, tol)
-    assert left(ws) == [B]
+    assert left(ws) == [B if feedback else 0]
     assert np.array_equal(st.cpu().numpy(), ref[3]) and np.array_equal(t.cpu().numpy(), ref[1])
     assert rel_error(out.cpu().numpy()[:, 3:3 + m], ref[0][:, 3:3 + m], 1e-12).max() <= BOUND[form]
 
