@@ -120,6 +120,6 @@ inline bool lane_has_shape(LaneForm form, int shape) { return form != LANE_AERO 
 const void* lane_kernel(int shape, LaneForm form);
 cudaError_t launch_lanes(const LaneParams& P, int shape, LaneForm form, int grid, cudaStream_t stream);
 // Doubles per sample of the aerosol problem's own section.
-inline int lane_aero_doubles(const AeroDev& A) { return 4 * A.nS + 6 * A.nP + 4 * A.nP * A.nS; }
+inline int lane_aero_doubles(const AeroDev& A) { return 4 * A.nS + 6 * A.nP + 4 * A.nP * A.nS + A.nP * A.nA; }
 
 }  // namespace tchem_gb

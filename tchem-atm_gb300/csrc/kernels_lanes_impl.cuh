@@ -708,11 +708,25 @@ struct Kernel {
   // The section holds, per sample: simc [nS][4] (accommodation coefficient, mean free path, partitioning
   // constant, kg m-3 -> ppm), nc [nP], part [nP][5] (radius, mean molecular weight, mass, moles, r / 3V),
   // tr [nP nS][4] (condensation coefficient, and the factors of 1 / density, 1 / molecular weight and the
-  // entry's own species in the transfer's derivative by a species of the particle).
+  // entry's own species in the transfer's derivative by a species of the particle), unit [nP nA].
+  //
+  // unit: what one kg m-3 in a particle is in the gas phase, number concentration x kg m-3 -> ppm of the species' own
+  // molecular weight, as a power of two. The matrix is that of the scaled unknowns: a bound on multipliers means
+  // nothing between rows in kg m-3 and rows in ppm, which are 1e5 and more apart, and powers of two leave every
+  // digit of the factors as it was.
   __device__ __forceinline__ double* ext(int i) const { return reinterpret_cast<double*>(sm + K.s.ext) + i * S + s; }
   __device__ __forceinline__ int nc_at() const { return 4 * K.aero.nS; }
   __device__ __forceinline__ int part_at() const { return 4 * K.aero.nS + K.aero.nP; }
   __device__ __forceinline__ int tr_at() const { return 4 * K.aero.nS + 6 * K.aero.nP; }
+  __device__ __forceinline__ int unit_at() const { return tr_at() + 4 * K.aero.nP * K.aero.nS; }
+  // 1 / u for a power of two
+  static __device__ __forceinline__ double inverse_unit(double u) {
+    return __longlong_as_double(0x7fe0000000000000ll - __double_as_longlong(u));
+  }
+  static __device__ __forceinline__ double power_of_two_below(double v) {
+    const int e = (__double2hiint(v) >> 20) & 0x7ff;  // 0, subnormal, infinite, NaN: no scaling
+    return __hiloint2double((e < 1023 - 300 || e > 1023 + 300 ? 1023 : e) << 20, 0);
+  }
 
   // Temperature and pressure terms and number concentrations of the new sample in lane c, by all threads.
   __device__ __forceinline__ void aero_setup_sample(int c, int smp, double p, double Tk) const {
@@ -725,6 +739,9 @@ struct Kernel {
     }
     for (int ip = threadIdx.x; ip < A.nP; ip += NT)
       e[(nc_at() + ip) * S] = K.number_conc[static_cast<size_t>(smp) * A.nP + ip];
+    for (int i = threadIdx.x; i < A.nP * A.nA; i += NT)
+      e[(unit_at() + i) * S] = power_of_two_below(K.number_conc[static_cast<size_t>(smp) * A.nP + i / A.nA] *
+                                                  (fp64::kAeroRuniv / A.mw[i % A.nA] * 1.0e6 * Tk / p));
   }
   __device__ __forceinline__ double ode(int i) const { return xs()[__ldg(K.p.pos + i) * S]; }
 
@@ -787,13 +804,15 @@ struct Kernel {
     T* d = ds() + (K.p.D - 2 * A.nP * A.nS * (1 + A.nA)) * S;
     for (int i = slot; i < A.nP * A.nS * (1 + A.nA); i += P) {
       const int e = i / (1 + A.nA), c = i - e * (1 + A.nA), ip = e / A.nS, is = e - ip * A.nS, t = tr_at() + 4 * e;
+      const int own = A.sim_idx[3 * is] - A.m_gas;
       double v = *ext(t);
       if (c > 0) {
         v = *ext(t + 1) / A.density[c - 1] + *ext(t + 2) / A.mw[c - 1];
-        if (A.sim_idx[3 * is] - A.m_gas == c - 1) v += *ext(t + 3);
+        if (own == c - 1) v += *ext(t + 3);
+        v *= inverse_unit(*ext(unit_at() + ip * A.nA + c - 1));
       }
       d[2 * i * S] = -*ext(nc_at() + ip) * v;
-      d[(2 * i + 1) * S] = v / *ext(4 * is + 3);
+      d[(2 * i + 1) * S] = v / *ext(4 * is + 3) * *ext(unit_at() + ip * A.nA + own);
     }
   }
 
@@ -921,10 +940,20 @@ struct Kernel {
     auto has = [&](int k) { return (sps[k] & 0xffff) < mm; };
     // the iterate itself is x
     double yn[NPS], fn[NPS], fg[NPS], rv[NPS], keff[NRS];
+    [[maybe_unused]] double unit[NPS] = {};  // of the slot's rows (gas species: 1)
+    auto to_matrix = [&](int k, double v) {
+      if constexpr (AERO) v *= unit[k];
+      return v;
+    };
+    auto from_matrix = [&](int k, double v) {
+      if constexpr (AERO) v *= inverse_unit(unit[k]);
+      return v;
+    };
     T kt[NRS];
 #pragma unroll
     for (int k = 0; k < NPS; ++k) {
       yn[k] = fn[k] = fg[k] = rv[k] = 0.0;
+      if constexpr (AERO) unit[k] = 1.0;
       if (has(k)) xs()[pos(k) * S] = 0.0;
     }
 #pragma unroll
@@ -1055,6 +1084,7 @@ struct Kernel {
           for (int k = 0; k < NPS; ++k) {
             yn[k] = has(k) ? row[column(k)] : 0.0;
             if (has(k)) xs()[pos(k) * S] = yn[k];
+            if constexpr (AERO) unit[k] = has(k) && species(k) >= mg ? *ext(unit_at() + species(k) - mg) : 1.0;
             fn[k] = fg[k] = rv[k] = 0.0;
           }
           if (A.keff_in) srcp = A.src_in + smp * A.src_stride;
@@ -1099,7 +1129,7 @@ struct Kernel {
         for (int k = 0; k < NPS; ++k)
           if (has(k)) {
             const double est = code == C_STEP ? 2.0 * kappa * dt * (e0 * fn[k] + e1 * fg[k] + e2 * f[k]) : 0.0;
-            lu()[zbase + pos(k) * S] = static_cast<T>(est);
+            lu()[zbase + pos(k) * S] = static_cast<T>(to_matrix(k, est));
           }
         __syncthreads();
         solve();
@@ -1110,7 +1140,7 @@ struct Kernel {
 #pragma unroll
           for (int k = 0; k < NPS; ++k)
             if (has(k)) {
-              const double est = fabs(static_cast<double>(lu()[zbase + pos(k) * S]));
+              const double est = fabs(from_matrix(k, static_cast<double>(lu()[zbase + pos(k) * S])));
               const double2 tol = reinterpret_cast<const double2*>(sm + K.s.tol)[pos(k)];
               const double wgt = tol.x + tol.y * fmax(fabs(yn[k]), fabs(xs()[pos(k) * S]));
               if (est * den > num * wgt) {
@@ -1269,7 +1299,7 @@ struct Kernel {
         if (has(k)) {
           const double y = xs()[pos(k) * S];
           g[k] = -((y - coef * f[k]) - rv[k]);
-          lu()[zbase + pos(k) * S] = static_cast<T>(g[k]);
+          lu()[zbase + pos(k) * S] = static_cast<T>(to_matrix(k, g[k]));
           if (kRefine) xt()[pos(k) * S] = static_cast<T>(y);
         }
       }
@@ -1303,7 +1333,7 @@ struct Kernel {
       if (bad) ci(I_BAD, s) = 1;
       solve();
 #pragma unroll
-      for (int k = 0; k < NPS; ++k) dx[k] = has(k) ? static_cast<double>(lu()[zbase + pos(k) * S]) : 0.0;
+      for (int k = 0; k < NPS; ++k) dx[k] = has(k) ? from_matrix(k, static_cast<double>(lu()[zbase + pos(k) * S])) : 0.0;
       if constexpr (kRefine) {
         // FP64 residual of (I - c J) dx = g, correction through the FP32 factors
 #pragma unroll

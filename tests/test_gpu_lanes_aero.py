@@ -72,6 +72,22 @@ def test_every_shape_equals_one_cell_per_cta(particles, B):
         assert compare_tchem(out[s, 3:], one[0][:, 3:]) <= 1e-9
 
 
+# Steps of seconds, where the entries between rows in kg m-3 and in ppm are 1e5 and more: no cell needs pivoting, so none is
+# left to the general kernel. Bound as for the perturbed batches over 100 s: 1e-8 in the reference's norms.
+@pytest.mark.parametrize("case,particles", [("simpol", 1), ("simpol", 30), ("cb05", 1), ("cb05", 3)])
+def test_no_cell_is_left_for_its_units(case, particles):
+    km, am, gas, parts = models(case)
+    am.set_number_of_particles(particles)
+    state, nc = perturbed(km, am, gas, parts, 5, 2)
+    tadv = time_advance_array(5, tend=30.0, dt=1e-6, dtmin=1e-20, dtmax=10.0, max_num_newton_iterations=20,
+                              num_time_iterations_per_interval=100000)
+    tol = np.tile([1e-12, 1e-6], (am.n_ode, 1))
+    out, t, status, st, left = advance(km, am, tadv, state, nc, tol)
+    ref, t_ref, _, status_ref, st_ref = AerosolOracle(km, am).time_advance(tadv, state, nc, TN, tol)
+    assert left == 0 and np.array_equal(status, status_ref) and np.array_equal(t, t_ref)
+    assert compare_tchem(out[:, 3:], ref[:, 3:]) <= 1e-8
+
+
 # Few particles of 1e-18 to 1e-16 kg grow by orders of magnitude within a step, so the first attempts are rejected, and
 # the Newton test, on the norm of the gas, ends each stage after one iteration: what the matrix holds for the particles
 # goes straight into the result. Bound: the oracle's difference Jacobian is within 1e-8 of the exact one, over the twelve
