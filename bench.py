@@ -884,7 +884,8 @@ def engine_arm(args, world: int, rank: int, local: int):
                      "fp32": {"achieved": ach32, "peak": peak32.value / 1e12,
                               "frac": ach32 / (peak32.value / 1e12)},
                      "note": "algorithmic FP64 flops count the right-hand sides only (the work formula); "
-                             "the FP32 side counts factorizations, solves and Jacobians"},
+                             "the FP32 side counts factorizations, solves and Jacobians as the dense "
+                             "algorithm's, which the sparse LU does not execute"},
     }
 
     if not args.no_e2e:

@@ -307,7 +307,8 @@ int tchem_gb_time_advance_hostbuf(const tchem_gb_mech* const* mechs, int n_mechs
  * itself and may allocate then. CUDA also places a kernel's code on the device at its first
  * launch (lazy module loading, the default): callers that must see no allocation at all include one
  * tchem_gb_time_advance call with the same mechanisms and form in their set-up (or run with
- * CUDA_MODULE_LOADING=EAGER). Make the set-up calls before any stream capture. All calls share
+ * CUDA_MODULE_LOADING=EAGER); the kernel goes by the batch size, so that call has the batch sizes
+ * used later. Make the set-up calls before any stream capture. All calls share
  * the array: calls that overlap on the GPU race and must be serialised. Device-side wait timeouts
  * are not reported through tchem_gb_device_error; samples no kernel reached keep the caller's
  * status value. */
@@ -433,12 +434,13 @@ int tchem_gb_e3sm_time_advance(const tchem_gb_mech* mech, int nbatch, const doub
  * TChem::AerosolChemistry::runDeviceBatch (src/core/TChem_AerosolChemistry.hpp:87-103,
  * src/core/TChem_AerosolChemistry.cpp:30-172, 236-260): TR-BDF2 on the ODE vector [active gas,
  * particle 0's aerosol species, particle 1's, ...] of M = m + nParticles * nSpec entries, with one
- * gas mechanism (box-model rate forms) and one aerosol model per call; plain FP64 form, one warp
- * per sample, device arrays, stream-ordered.
+ * gas mechanism (box-model rate forms) and one aerosol model per call; plain FP64 form, device arrays,
+ * stream-ordered.
  *   tol_time[M][2]; number_conc[nbatch][nParticles]; state and state_out rows [rho, p, T, active
  *   gas, constant gas, particles] of width 3 + nSpec + nParticles * nSpec_aerosol (may alias).
- * The Newton Jacobian is a forward difference of the RHS, column j with the step
- * 1e-8 max(|y_j|, 1e-20) (the reference's computeJacobian); fac, the reference's per-sample
+ * The Newton Jacobian is analytic (batched sparse LU); a sample left to the general kernel (Jacobian interval above 1,
+ * pivoting needed, or more than shared memory holds) takes a forward difference of the RHS, column j with the step
+ * 1e-8 max(|y_j|, 1e-20) (the reference's computeJacobian). fac, the reference's per-sample
  * difference factors, may be NULL and is not read. rho, p, T and the constant gas species are
  * copied through. Refused with TCHEM_GB_ERR_UNSUPPORTED: a SIMPOL entry whose gas species is a
  * constant species, M above 320, or rate forms outside the box model's. The workspace holds the

@@ -21,9 +21,9 @@
 // 104 k with 16. FP32 with 16 samples: solves 21 k, tail 24 k, sparse factorization 12 k, matrix 11 k,
 // right-hand side 9 k, residual product 10 k, error test and norms 16 k. Measured against the dense kernels
 // (one GB300): 51 species, one sample over 60 s 93 ms to 54 ms, 4,096 samples over 3,600 s 1.20 s to 1.03 s (FP32), 300 samples
-// over 0.1 s 1.02 s to 204 ms (FP64); 120 species, 257 samples over 1 s 451 ms to 213 ms; 300 species, 24 samples over
+// over 0.1 s 1.02 s to 178 ms (FP64); 120 species, 257 samples over 1 s 451 ms to 213 ms; 300 species, 24 samples over
 // 1e-4 s 443 ms to 75 ms (the blocked LU on tensor cores with the matrix in L2); E3SM, 2,000 columns over 1,800 s
-// 118 ms to 8.5 ms (FP64).
+// 118 ms to 8.5 ms (FP64). Where a register kernel is the faster one: lanes_pay_for_box in lane_tables.cu.
 //
 // T = float: the full-Newton FP32 form (FP32 matrix, factors and solves, FP64 residual, one
 // refinement sweep with an FP64 Jacobian-vector product per solve). T = double: the plain form.

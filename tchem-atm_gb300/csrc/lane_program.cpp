@@ -318,8 +318,11 @@ int lane_entries(const LanePattern& pat, int P, int n_t) {
 
 // By the estimated cycles of one round's factorization and solves. Issue: a packet row is about 35
 // instructions over four schedulers; latency: a level's barrier and dependent loads about 250 cycles, a
-// tail step about 250. FP64 has no tail: the inverse needs three times the products of the triangular
-// factors, on a pipe of 2 per cycle.
+// tail pivot about 250 (measured with one pivot per step; steps take two now, which these choices do not use yet). The
+// tables' size, not known before the program is built, is taken as 2,048 bytes, and as 704 with two CTAs per SM, what the
+// 51-species sections leave there at a tail of 24; the program's own size is checked before a shape is offered. FP64
+// has no tail: the inverse needs three times the products of the triangular factors, on a pipe of 2 per cycle (measured
+// with 16 samples per CTA; with one the pipe idles, and a tail there has not been tried).
 int lane_tail_size(const LaneInput& in, const LanePattern& pat, const LaneShape& shape, bool fp64) {
   if (fp64) return 0;
   const int S = shape.S, warps = shape.warps;

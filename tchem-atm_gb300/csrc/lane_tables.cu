@@ -169,15 +169,17 @@ LaneTables* upload_aero_lane_tables(const HostTables& ht, const AeroDev& A, cons
 // sample, the shortest round) whose lanes hold the batch at once, or `slack` times over, else the most
 // that one CTA per SM holds (samples then follow each other through the lanes). Box samples differ in length, the
 // longest taking about twice the mean, and the longest one's rounds are shorter with fewer samples beside it:
-// FP32 with up to 64 species gains up to twice the room (51 species over 2 s: 1,893 samples 232 ms with
-// 16 per CTA and 217 with 8, 1,230 samples 219 and 154, 230 samples 104 with two and 92 with one; 310 samples 93 with
-// two and 100 with one), where a round's time depends on the samples in it more than that (FP64, larger matrices) up to
-// three times (51 species FP64, 900 samples 155 ms with four and 141 with two; 120 species, 400 samples 144 ms with
-// two and 131 with one). E3SM columns and aerosol cells are alike in length and are held at once (FP64, 1,300
-// columns over 600 s: 12 ms with 8, 8 with 16). The shape with two CTAs per SM takes longer per
-// round (51 species: 160 k cycles for 32 samples against 104 k for 16) and less per sample, so it pays
-// when its lanes are filled several times over, from four times its room: 10,000 samples over 1 s 464 ms
-// with one CTA per SM, 494 ms with two; 16,384 695 and 690 ms; 40,000 1,462 and 1,343 ms.
+// FP32 with up to 64 species gains up to twice the room (51 species over 2 s: 2,432 samples 269 ms with
+// 16 per CTA and 257 with 8, 620 samples 149 with two and 133 with four, 230 samples 104 with two and 92 with one; 310
+// samples 93 with two and 100 with one), where a round's time depends on the samples in it more than that (FP64, larger
+// matrices) up to three times (51 species FP64, 900 samples 155 ms with four and 141 with two; 120 species, 400 samples
+// 144 ms with two and 131 with one; other sizes in between were not measured). E3SM columns and aerosol cells are alike
+// in length and are held at once (FP64, 1,300 columns over 600 s: 12 ms with 8, 8 with 16). The shape with two CTAs per
+// SM takes longer per round (51 species: 160 k cycles for 32 samples against 104 k for 16) and less per sample, so for
+// boxes it pays when its lanes are filled several times over, from four times its room: 10,000 samples over 1 s 464 ms
+// with one CTA per SM, 494 ms with two; 16,384 695 and 690 ms; 40,000 1,462 and 1,343 ms. E3SM columns follow the
+// same line, though alike in length they would gain from it as soon as one CTA per SM does not hold them (FP64 over 600 s,
+// 2,600 columns 14.7 ms with one CTA and 10.2 with two, 4,000 15.1 and 10.6).
 LanePlan plan_lanes(const LaneTables* t, LaneForm form, int ext, int sm_count, int max_smem, int nbatch, int slack) {
   LanePlan p;
   p.form = form;
